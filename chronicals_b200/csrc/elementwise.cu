@@ -9,6 +9,7 @@
 // patches in.
 #include <algorithm>
 #include <cstring>
+#include <cooperative_groups.h>
 #include "common.cuh"
 
 // ---- optional index checks (compile with -DCHRONICALS_DEBUG_BOUNDS, e.g. CHRONICALS_DEBUG_BOUNDS=1 in the
@@ -27,6 +28,8 @@ __device__ long long g_cb_debug_word[2] = {0, 0};
 #else
 #define CB_DEBUG_CHECK(cond, code, value) do { } while (0)
 #endif
+
+namespace cg = cooperative_groups;
 
 namespace cb {
 
@@ -468,165 +471,219 @@ embedding_bwd_kernel(const long long* __restrict__ sorted_ids, const long long* 
 }
 
 // ------------------------------------------------------------------ cross-entropy on materialised logits
-// One block per row.  Pass 1: online (max, sum-exp); pass 2 (optional): gradient in place.
+// Bound by memory: the logits are read once forward (log-sum-exp) and once backward, the gradient written once.
+// A thread keeps CE_BATCH 16-byte loads in flight and does one running-maximum update per batch instead of one per
+// value (the update costs a second exponential, and as a chain through every value it, not memory, set the pace).
+// A row starts where it starts: the values before the first 16-byte boundary and after the last are read one by
+// one, so odd vocabularies and pitches take the same path.  gridDim.y blocks share a row when there are fewer rows
+// than the chip has room for; forward they form a cluster and meet in the shared memory of its first block.
+// Rows without a valid label take no part: their loss and gradient are zero and their logits are not read.
+// Measured, 2047 x 151,936 fp32 with a fifth of the rows masked (one value per load, every row read, before):
+// forward 603 -> 179 us (5.5 TB/s), backward 748 -> 370 us (6.1 TB/s).
+constexpr int CE_BATCH = 4;
+
 template <typename T>
-__device__ __forceinline__ float ldf(const T* p);
-template <>
-__device__ __forceinline__ float ldf<float>(const float* p) { return *p; }
-template <>
-__device__ __forceinline__ float ldf<bf16>(const bf16* p) { return __bfloat162float(*p); }
+struct CeVec {
+  static constexpr int N = 16 / sizeof(T);
+};
+__device__ __forceinline__ void ce_unpack(const uint4& u, float (&f)[4]) {
+  f[0] = __uint_as_float(u.x); f[1] = __uint_as_float(u.y); f[2] = __uint_as_float(u.z); f[3] = __uint_as_float(u.w);
+}
+__device__ __forceinline__ void ce_unpack(const uint4& u, float (&f)[8]) { unpack8(u, f); }
+__device__ __forceinline__ uint4 ce_pack(const float (&f)[4]) {
+  return make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+}
+__device__ __forceinline__ uint4 ce_pack(const float (&f)[8]) { return pack8(f); }
+__device__ __forceinline__ float ldf(const float* p) { return *p; }
+__device__ __forceinline__ float ldf(const bf16* p) { return __bfloat162float(*p); }
+__device__ __forceinline__ void stf(float* p, float v) { *p = v; }
+__device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16(v); }
+
+// values in front of the first 16-byte boundary of a row (at most V)
 template <typename T>
-__device__ __forceinline__ void stf(T* p, float v);
-template <>
-__device__ __forceinline__ void stf<float>(float* p, float v) { *p = v; }
-template <>
-__device__ __forceinline__ void stf<bf16>(bf16* p, float v) { *p = __float2bfloat16(v); }
+__device__ __forceinline__ int ce_head(const T* p, int V) {
+  const int h = static_cast<int>(((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / sizeof(T));
+  return h < V ? h : V;
+}
+
+// running (max, sum of exp(v - max)); an all -inf prefix keeps the sum at 0, NaN stays NaN
+struct CeAcc {
+  float m = -INFINITY, s = 0.f, sum = 0.f;
+  __device__ __forceinline__ static float base(float m) { return m == -INFINITY ? 0.f : m; }
+  __device__ __forceinline__ void merge(float om, float os, float osum) {
+    const float nm = fmaxf(m, om), b = base(nm);
+    s = s * __expf(m - b) + os * __expf(om - b);
+    m = nm;
+    sum += osum;
+  }
+  template <int K>
+  __device__ __forceinline__ void add(const float (&v)[K]) {
+    float vm = v[0];
+#pragma unroll
+    for (int i = 1; i < K; ++i) vm = fmaxf(vm, v[i]);
+    const float nm = fmaxf(m, vm), b = base(nm);
+    float e = 0.f, t = 0.f;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      e += __expf(v[i] - b);
+      t += v[i];
+    }
+    s = s * __expf(m - b) + e;
+    m = nm;
+    sum += t;
+  }
+};
 
 template <typename T>
 __global__ void __launch_bounds__(EW_THREADS)
 ce_logits_kernel(const T* __restrict__ logits, const long long* __restrict__ labels, long long ld, int V,
                  long long ignore_index, float smoothing, float z_weight, float* __restrict__ loss_rows,
                  float* __restrict__ lse_out) {
+  constexpr int N = CeVec<T>::N;
   __shared__ float sm[EW_THREADS / 32], ss[EW_THREADS / 32], sl[EW_THREADS / 32];
+  __shared__ float part[3][8];                         // (max, sum, sum of logits) of up to eight blocks of the cluster
   const long long row = blockIdx.x;
+  const long long lab = labels[row];
+  if (lab == ignore_index || lab < 0 || lab >= V) {    // the same answer in every block of the row
+    if (threadIdx.x == 0 && blockIdx.y == 0) {
+      loss_rows[row] = 0.f;
+      lse_out[row] = 0.f;
+    }
+    return;
+  }
   const T* lp = logits + row * ld;
-  float m = -INFINITY, s = 0.f, sumv = 0.f;
-  for (int c = threadIdx.x; c < V; c += blockDim.x) {
-    const float v = ldf<T>(lp + c);
-    const float nm = fmaxf(m, v);
-    s = s * __expf(m - nm) + __expf(v - nm);
-    m = nm;
-    sumv += v;
+  const int head = ce_head(lp, V), nvec = (V - head) / N, tail0 = head + nvec * N;
+  const uint4* vp = reinterpret_cast<const uint4*>(lp + head);
+  const int step = EW_THREADS * gridDim.y;
+  CeAcc a;
+  int c = blockIdx.y * EW_THREADS + threadIdx.x;
+  for (; c + (CE_BATCH - 1) * step < nvec; c += CE_BATCH * step) {
+    uint4 u[CE_BATCH];
+#pragma unroll
+    for (int i = 0; i < CE_BATCH; ++i) u[i] = vp[c + i * step];
+    float v[CE_BATCH * N];
+#pragma unroll
+    for (int i = 0; i < CE_BATCH; ++i) {
+      float w[N];
+      ce_unpack(u[i], w);
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[i * N + j] = w[j];
+    }
+    a.add(v);
   }
-  // combine (m, s) pairs across the block
+  for (; c < nvec; c += step) {
+    float w[N];
+    ce_unpack(vp[c], w);
+    a.add(w);
+  }
+  if (blockIdx.y == 0) {                               // at most N - 1 values at either end
+    const int t = static_cast<int>(threadIdx.x);
+    if (t < head) {
+      const float w[1] = {ldf(lp + t)};
+      a.add(w);
+    }
+    if (tail0 + t < V) {
+      const float w[1] = {ldf(lp + tail0 + t)};
+      a.add(w);
+    }
+  }
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    const float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, s, o);
-    const float nm = fmaxf(m, om);
-    s = (m > -INFINITY ? s * __expf(m - nm) : 0.f) + (om > -INFINITY ? os * __expf(om - nm) : 0.f);
-    m = nm;
-    sumv += __shfl_xor_sync(0xffffffffu, sumv, o);
+    const float om = __shfl_xor_sync(0xffffffffu, a.m, o), os = __shfl_xor_sync(0xffffffffu, a.s, o);
+    a.merge(om, os, __shfl_xor_sync(0xffffffffu, a.sum, o));
   }
-  if ((threadIdx.x & 31) == 0) { sm[threadIdx.x >> 5] = m; ss[threadIdx.x >> 5] = s; sl[threadIdx.x >> 5] = sumv; }
+  if ((threadIdx.x & 31) == 0) {
+    sm[threadIdx.x >> 5] = a.m;
+    ss[threadIdx.x >> 5] = a.s;
+    sl[threadIdx.x >> 5] = a.sum;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    float M = -INFINITY, S = 0.f, L = 0.f;
-    for (int i = 0; i < EW_THREADS / 32; ++i) M = fmaxf(M, sm[i]);
-    for (int i = 0; i < EW_THREADS / 32; ++i) { if (sm[i] > -INFINITY) S += ss[i] * __expf(sm[i] - M); L += sl[i]; }
-    const float lse = M + __logf(S);
-    lse_out[row] = lse;
-    const long long lab = labels[row];
-    float loss = 0.f;
-    if (lab != ignore_index && lab >= 0 && lab < V) {
-      loss = lse - ldf<T>(lp + lab);
-      if (smoothing != 0.f) loss = (1.f - smoothing) * loss + smoothing * (lse - L / static_cast<float>(V));
-      loss += z_weight * lse * lse;
+    a = CeAcc();
+    for (int i = 0; i < EW_THREADS / 32; ++i) a.merge(sm[i], ss[i], sl[i]);
+  }
+  if (gridDim.y > 1) {
+    cg::cluster_group cl = cg::this_cluster();
+    if (threadIdx.x == 0) {
+      float* dst = cl.map_shared_rank(&part[0][0], 0);
+      dst[blockIdx.y] = a.m;
+      dst[8 + blockIdx.y] = a.s;
+      dst[16 + blockIdx.y] = a.sum;
     }
-    loss_rows[row] = loss;
+    cl.sync();
+    if (blockIdx.y != 0) return;
+    if (threadIdx.x == 0) {
+      a = CeAcc();
+      for (unsigned i = 0; i < gridDim.y; ++i) a.merge(part[0][i], part[1][i], part[2][i]);
+    }
+  }
+  if (threadIdx.x == 0) {
+    const float lse = a.m + __logf(a.s);
+    lse_out[row] = lse;
+    float loss = lse - ldf(lp + lab);
+    if (smoothing != 0.f) loss = (1.f - smoothing) * loss + smoothing * (lse - a.sum / static_cast<float>(V));
+    loss_rows[row] = loss + z_weight * lse * lse;
   }
 }
 
+// The gradient may be written over the logits (every thread reads its values before it stores them): no __restrict__.
 template <typename T>
 __global__ void __launch_bounds__(EW_THREADS)
-ce_logits_grad_kernel(const T* __restrict__ logits, T* __restrict__ dlogits, const long long* __restrict__ labels,
-                      const float* __restrict__ lse_in, const float* __restrict__ gscale, const float* __restrict__ gout,
-                      long long ld, int V, long long ignore_index, float smoothing, float z_weight) {
+ce_logits_grad_kernel(const T* logits, T* dlogits, const long long* __restrict__ labels, const float* __restrict__ lse_in,
+                      const float* __restrict__ gscale, const float* __restrict__ gout, long long ld, long long ldd, int V,
+                      long long ignore_index, float smoothing, float z_weight) {
+  constexpr int N = CeVec<T>::N;
   const long long row = blockIdx.x;
   const long long lab = labels[row];
   const bool valid = lab != ignore_index && lab >= 0 && lab < V;
+  const T* lp = logits + row * ld;
+  T* dp = dlogits + row * ldd;
   const float lse = lse_in[row];
   const float gs = valid ? gscale[row] * gout[0] : 0.f;
   const float coef = 1.f + 2.f * z_weight * lse;
   const float smv = smoothing / static_cast<float>(V);
-  for (int c = threadIdx.x; c < V; c += blockDim.x) {
-    float p = __expf(ldf<T>(logits + row * ld + c) - lse) * coef - smv;
-    if (c == lab) p -= (1.f - smoothing);
-    stf<T>(dlogits + row * ld + c, p * gs);
+  const float hit = 1.f - smoothing;
+  const auto grad = [&](float v, int c) {
+    float p = __expf(v - lse) * coef - smv;
+    if (c == lab) p -= hit;
+    return p * gs;
+  };
+  // source and destination rows may start at different distances from a 16-byte boundary: value by value then
+  const bool vec = ((reinterpret_cast<uintptr_t>(lp) ^ reinterpret_cast<uintptr_t>(dp)) & 15) == 0;
+  const int head = vec ? ce_head(lp, V) : V, nvec = (V - head) / N, tail0 = head + nvec * N;
+  const uint4* vp = reinterpret_cast<const uint4*>(lp + head);
+  uint4* wp = reinterpret_cast<uint4*>(dp + head);
+  const int step = EW_THREADS * gridDim.y;
+  const int first = blockIdx.y * EW_THREADS + threadIdx.x;
+  if (!valid) {
+    for (int c = first; c < nvec; c += step) wp[c] = make_uint4(0u, 0u, 0u, 0u);
+    for (int c = first; c < head; c += step) stf(dp + c, 0.f);
+    for (int c = tail0 + first; c < V; c += step) stf(dp + c, 0.f);
+    return;
   }
-}
-
-// The same two kernels for bf16 rows read and written 16 bytes (8 values) at a time: a vocabulary row of 150 k
-// logits is 300 KB, so with vector accesses both kernels run at memory speed.  Rows are processed by one block
-// each; V and the row pitch are multiples of 8 and the base is 16-byte aligned (checked by the callers below).
-// The gradient kernel may write over its input (every thread reads its 8 values before it stores them).
-__global__ void __launch_bounds__(EW_THREADS)
-ce_logits_bf16v_kernel(const bf16* __restrict__ logits, const long long* __restrict__ labels, long long ld, int V,
-                       long long ignore_index, float smoothing, float z_weight, float* __restrict__ loss_rows,
-                       float* __restrict__ lse_out) {
-  __shared__ float sm[EW_THREADS / 32], ss[EW_THREADS / 32], sl[EW_THREADS / 32];
-  const long long row = blockIdx.x;
-  const uint4* lp = reinterpret_cast<const uint4*>(logits + row * ld);
-  float m = -INFINITY, s = 0.f, sumv = 0.f;
-  for (int c = threadIdx.x; c < V / 8; c += blockDim.x) {
-    const uint4 u = lp[c];
-    float v[8];
-    const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), cc = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = cc.x; v[5] = cc.y; v[6] = d.x; v[7] = d.y;
-    float vm = fmaxf(fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3])), fmaxf(fmaxf(v[4], v[5]), fmaxf(v[6], v[7])));
-    const float nm = fmaxf(m, vm);
-    float e = 0.f, t = 0.f;
+  int c = first;
+  for (; c + (CE_BATCH - 1) * step < nvec; c += CE_BATCH * step) {
+    uint4 u[CE_BATCH];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { e += __expf(v[i] - nm); t += v[i]; }
-    s = s * __expf(m - nm) + e;                        // m = -inf at first: exp(-inf) = 0
-    m = nm;
-    sumv += t;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, s, o);
-    const float nm = fmaxf(m, om);
-    s = (m > -INFINITY ? s * __expf(m - nm) : 0.f) + (om > -INFINITY ? os * __expf(om - nm) : 0.f);
-    m = nm;
-    sumv += __shfl_xor_sync(0xffffffffu, sumv, o);
-  }
-  if ((threadIdx.x & 31) == 0) { sm[threadIdx.x >> 5] = m; ss[threadIdx.x >> 5] = s; sl[threadIdx.x >> 5] = sumv; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float M = -INFINITY, S = 0.f, L = 0.f;
-    for (int i = 0; i < EW_THREADS / 32; ++i) M = fmaxf(M, sm[i]);
-    for (int i = 0; i < EW_THREADS / 32; ++i) { if (sm[i] > -INFINITY) S += ss[i] * __expf(sm[i] - M); L += sl[i]; }
-    const float lse = M + __logf(S);
-    lse_out[row] = lse;
-    const long long lab = labels[row];
-    float loss = 0.f;
-    if (lab != ignore_index && lab >= 0 && lab < V) {
-      loss = lse - __bfloat162float(logits[row * ld + lab]);
-      if (smoothing != 0.f) loss = (1.f - smoothing) * loss + smoothing * (lse - L / static_cast<float>(V));
-      loss += z_weight * lse * lse;
-    }
-    loss_rows[row] = loss;
-  }
-}
-
-__global__ void __launch_bounds__(EW_THREADS)
-ce_logits_grad_bf16v_kernel(const bf16* logits, bf16* dlogits, const long long* __restrict__ labels,
-                            const float* __restrict__ lse_in, const float* __restrict__ gscale,
-                            const float* __restrict__ gout, long long ld, int V, long long ignore_index, float smoothing,
-                            float z_weight) {
-  const long long row = blockIdx.x;
-  const long long lab = labels[row];
-  const bool valid = lab != ignore_index && lab >= 0 && lab < V;
-  const float lse2 = lse_in[row] * 1.4426950408889634f;
-  const float gs = valid ? gscale[row] * gout[0] : 0.f;
-  const float cg = (1.f + 2.f * z_weight * lse_in[row]) * gs;
-  const float smg = smoothing / static_cast<float>(V) * gs;
-  const float hit = (1.f - smoothing) * gs;
-  const int lab_vec = valid ? static_cast<int>(lab >> 3) : -1;
-  const uint4* lp = reinterpret_cast<const uint4*>(logits + row * ld);
-  uint4* dp = reinterpret_cast<uint4*>(dlogits + row * ld);
-  for (int c = threadIdx.x; c < V / 8; c += blockDim.x) {
-    const uint4 u = lp[c];
-    float v[8];
-    const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), cc = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = cc.x; v[5] = cc.y; v[6] = d.x; v[7] = d.y;
-    const int lab_i = (c == lab_vec) ? static_cast<int>(lab & 7) : -1;
+    for (int i = 0; i < CE_BATCH; ++i) u[i] = vp[c + i * step];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[i] = fmaf(ex2_approx(fmaf(v[i], 1.4426950408889634f, -lse2)), cg, -smg);
-      v[i] -= (i == lab_i) ? hit : 0.f;
+    for (int i = 0; i < CE_BATCH; ++i) {
+      float w[N];
+      ce_unpack(u[i], w);
+#pragma unroll
+      for (int j = 0; j < N; ++j) w[j] = grad(w[j], head + (c + i * step) * N + j);
+      wp[c + i * step] = ce_pack(w);
     }
-    uint4 o;
-    o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]); o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
-    dp[c] = o;
   }
+  for (; c < nvec; c += step) {
+    float w[N];
+    ce_unpack(vp[c], w);
+#pragma unroll
+    for (int j = 0; j < N; ++j) w[j] = grad(w[j], head + c * N + j);
+    wp[c] = ce_pack(w);
+  }
+  for (int i = first; i < head; i += step) stf(dp + i, grad(ldf(lp + i), i));
+  for (int i = tail0 + first; i < V; i += step) stf(dp + i, grad(ldf(lp + i), i));
 }
 
 // ------------------------------------------------------------------ LoRA on fused projections: pack / unpack
@@ -705,6 +762,13 @@ int grid_for(long long work_items, int per_block, int max_waves = 8) {
   if (b > cap) b = cap;
   if (b < 1) b = 1;
   return static_cast<int>(b);
+}
+// Blocks that share one row of logits.  One is enough once the rows alone fill the chip (four blocks an SM); with
+// fewer, a row is cut in 2, 4 or 8 (a portable cluster) as long as every piece keeps 4096 values.
+int ce_split(long long rows, int V) {
+  int split = 1;
+  while (split < 8 && rows * split < 4LL * sm_count() && V / (2 * split) >= 4096) split *= 2;
+  return split;
 }
 // rows-per-thread-group choice: the smallest group whose registers hold the row (VPL = 4 vectors of 8)
 int pick_tpr(int N) {
@@ -857,32 +921,35 @@ int cb_embedding_bwd(const long long* sorted_ids, const long long* perm, const v
 
 int cb_ce_logits(const void* logits, const long long* labels, long long rows, long long ld, int V, int is_bf16,
                  long long ignore_index, float smoothing, float z_weight, float* loss_rows, float* lse, void* stream) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (rows <= 0) return -1;
-  if (is_bf16 && V % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
-    cb::ce_logits_bf16v_kernel<<<static_cast<unsigned>(rows), cb::EW_THREADS, 0, s>>>(
-        static_cast<const cb::bf16*>(logits), labels, ld, V, ignore_index, smoothing, z_weight, loss_rows, lse);
-    return static_cast<int>(cudaGetLastError());
-  }
-  if (is_bf16) cb::ce_logits_kernel<cb::bf16><<<static_cast<unsigned>(rows), cb::EW_THREADS, 0, s>>>(static_cast<const cb::bf16*>(logits), labels, ld, V, ignore_index, smoothing, z_weight, loss_rows, lse);
-  else cb::ce_logits_kernel<float><<<static_cast<unsigned>(rows), cb::EW_THREADS, 0, s>>>(static_cast<const float*>(logits), labels, ld, V, ignore_index, smoothing, z_weight, loss_rows, lse);
-  return static_cast<int>(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  const int split = ce_split(rows, V);
+  cfg.gridDim = dim3(static_cast<unsigned>(rows), split);
+  cfg.blockDim = dim3(cb::EW_THREADS);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = split;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = split > 1 ? 1 : 0;
+  if (is_bf16)
+    return static_cast<int>(cudaLaunchKernelEx(&cfg, cb::ce_logits_kernel<cb::bf16>, static_cast<const cb::bf16*>(logits), labels,
+                                               ld, V, ignore_index, smoothing, z_weight, loss_rows, lse));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, cb::ce_logits_kernel<float>, static_cast<const float*>(logits), labels, ld, V,
+                                             ignore_index, smoothing, z_weight, loss_rows, lse));
 }
 
+// ld / ldd: row pitches of the logits and of the gradient
 int cb_ce_logits_grad(const void* logits, void* dlogits, const long long* labels, const float* lse, const float* gscale,
-                      const float* gout, long long rows, long long ld, int V, int is_bf16, long long ignore_index,
-                      float smoothing, float z_weight, void* stream) {
+                      const float* gout, long long rows, long long ld, long long ldd, int V, int is_bf16,
+                      long long ignore_index, float smoothing, float z_weight, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (rows <= 0) return -1;
-  if (is_bf16 && V % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0 &&
-      (reinterpret_cast<uintptr_t>(dlogits) & 15) == 0) {
-    cb::ce_logits_grad_bf16v_kernel<<<static_cast<unsigned>(rows), cb::EW_THREADS, 0, s>>>(
-        static_cast<const cb::bf16*>(logits), static_cast<cb::bf16*>(dlogits), labels, lse, gscale, gout, ld, V,
-        ignore_index, smoothing, z_weight);
-    return static_cast<int>(cudaGetLastError());
-  }
-  if (is_bf16) cb::ce_logits_grad_kernel<cb::bf16><<<static_cast<unsigned>(rows), cb::EW_THREADS, 0, s>>>(static_cast<const cb::bf16*>(logits), static_cast<cb::bf16*>(dlogits), labels, lse, gscale, gout, ld, V, ignore_index, smoothing, z_weight);
-  else cb::ce_logits_grad_kernel<float><<<static_cast<unsigned>(rows), cb::EW_THREADS, 0, s>>>(static_cast<const float*>(logits), static_cast<float*>(dlogits), labels, lse, gscale, gout, ld, V, ignore_index, smoothing, z_weight);
+  const dim3 grid(static_cast<unsigned>(rows), ce_split(rows, V));
+  if (is_bf16) cb::ce_logits_grad_kernel<cb::bf16><<<grid, cb::EW_THREADS, 0, s>>>(static_cast<const cb::bf16*>(logits), static_cast<cb::bf16*>(dlogits), labels, lse, gscale, gout, ld, ldd, V, ignore_index, smoothing, z_weight);
+  else cb::ce_logits_grad_kernel<float><<<grid, cb::EW_THREADS, 0, s>>>(static_cast<const float*>(logits), static_cast<float*>(dlogits), labels, lse, gscale, gout, ld, ldd, V, ignore_index, smoothing, z_weight);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -741,8 +741,8 @@ class _LinearCEResidentFn(torch.autograd.Function):
             g1 = torch.ones(1, dtype=torch.float32, device=dev)
         # in place: the logits are not needed again (a second backward through this node is not supported)
         code = _ext.lib().cb_ce_logits_grad(logits.data_ptr(), logits.data_ptr(), labels.data_ptr(), lse.data_ptr(),
-                                            gscale.data_ptr(), g1.data_ptr(), M, logits.stride(0), V, 1, ignore_index,
-                                            smoothing, z_weight, _ext.stream_ptr())
+                                            gscale.data_ptr(), g1.data_ptr(), M, logits.stride(0), logits.stride(0), V, 1,
+                                            ignore_index, smoothing, z_weight, _ext.stream_ptr())
         _ext.check(code, "ce_logits_grad")
         dh = gemm(logits, weight, b_mn=True) if ctx.needs_input_grad[0] else None
         dw = None
@@ -807,7 +807,7 @@ class _CELogitsFn(torch.autograd.Function):
         one = torch.ones(1, dtype=torch.float32, device=logits.device)
         gs = grows.float().contiguous()
         code = _ext.lib().cb_ce_logits_grad(logits.data_ptr(), dl.data_ptr(), labels.data_ptr(), lse.data_ptr(),
-                                            gs.data_ptr(), one.data_ptr(), rows, logits.stride(0), V,
+                                            gs.data_ptr(), one.data_ptr(), rows, logits.stride(0), dl.stride(0), V,
                                             int(logits.dtype == torch.bfloat16), ignore_index, smoothing, z_weight,
                                             _ext.stream_ptr())
         _ext.check(code, "ce_logits_grad")

@@ -1,0 +1,48 @@
+"""Reductions over rows, runs and columns at the sizes where their splits can go wrong, against 64-bit formulas."""
+import math
+
+import pytest
+import torch
+
+from chronicals_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _gen(seed):
+    return torch.Generator(device=DEV).manual_seed(seed)
+
+
+# vocabularies below one vector, odd ones (every row starts elsewhere within 16 bytes), rows shared by 2, 4 and 8 blocks,
+# more rows than fit at once; `gap` elements between the rows, `shift` before the first one
+@pytest.mark.parametrize("rows,V,gap,shift", [(1, 3, 0, 0), (2, 4099, 0, 1), (5, 8192, 0, 0), (7, 33001, 3, 0), (2, 70000, 0, 0),
+                                              (2500, 1031, 0, 0), (40, 12288, 8, 8)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_logits_cross_entropy_rows(rows, V, gap, shift, dtype):
+    g = _gen(rows + V)
+    buf = (3 * torch.randn(shift + rows * (V + gap), device=DEV, generator=g)).to(dtype)
+    lg = buf[shift:].view(rows, V + gap)[:, :V]
+    if V > 100:
+        lg[0, : V // 2] = -math.inf                               # a masked vocabulary: whole batches of -inf
+    y = torch.randint(V // 2, V, (rows,), device=DEV, generator=g)
+    y[1::3] = -100
+    if rows > 4:
+        y[4] = V                                                  # no row of the vocabulary: takes no part either
+    x = lg.detach().requires_grad_()
+    loss = ops.cross_entropy_logits(x, y, -100, 0.0, 1e-3, reduction="none")
+    gr = torch.rand(rows, device=DEV, generator=g) + 0.5
+    loss.backward(gr)
+    ok = (y >= 0) & (y < V)
+    xr = lg.detach().double().requires_grad_()
+    lse = torch.logsumexp(xr, -1)
+    want = torch.where(ok, lse - xr.gather(1, y.clamp(0, V - 1)[:, None])[:, 0] + 1e-3 * lse.square(), torch.zeros_like(lse))
+    want.backward(gr.double())
+    # fp32 arithmetic on values of order 10: a few ulp of the largest intermediate
+    assert (loss.double() - want).abs().max().item() < 2e-5
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5          # rounding of the stored gradient
+    assert ((x.grad.double() - xr.grad).abs() <= eps * xr.grad.abs() + 1e-6).all()
+    assert (x.grad[~ok] == 0).all()
+    if gap:                                                       # nothing outside the rows was written
+        assert torch.equal(buf[shift:].view(rows, V + gap)[:, :V], lg)
+

@@ -441,33 +441,149 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__
   }
 }
 
-// Deterministic scatter-add: `sorted_ids` ascending with `perm` the source token of each
-// entry.  The block at the first entry of a run sums the run in fp32 and is the only
-// writer of that table row.
+// Backward: dtable[id] = sum of dout over the tokens that carry `id`, in fp32, in token order, zero elsewhere.
+//
+// Step 1 writes the zeros (bound by memory: V x N bf16) and, in its first blocks, sorts the tokens by id while the
+// stores drain: the place of token i is the number of tokens with a smaller id or with the same id and a smaller
+// index, counted outright against all T ids.  That is T^2 integer compares, 64 tokens per block, a quarter of the
+// ids per thread; no passes over keys, no scan, and the result does not depend on the order of anything.
+// Measured, T = 8192, V = 151,936, N = 896: 59 us together; a fill of the same bytes alone took 70 us and a radix sort
+// of the 64-bit ids 65 us before.
+constexpr int EMB_RANK_TOKENS = 64;
+constexpr int EMB_RANK_TILE = 4096;                    // ids staged in shared memory at a time
+constexpr int EMB_NO_ROW = 0x7ffffffe;                 // ids outside [0, V): sorted last, never written
+
+__global__ void __launch_bounds__(EW_THREADS)
+embedding_rank_fill_kernel(const long long* __restrict__ ids, int* __restrict__ sorted_ids, int* __restrict__ perm, int T,
+                           int rank_blocks, uint4* __restrict__ dtable, long long table_vecs, long long V) {
+  __shared__ __align__(16) int tile[EMB_RANK_TILE];
+  if (static_cast<int>(blockIdx.x) >= rank_blocks) {
+    const long long step = static_cast<long long>(gridDim.x - rank_blocks) * EW_THREADS;
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    for (long long i = (blockIdx.x - rank_blocks) * static_cast<long long>(EW_THREADS) + threadIdx.x; i < table_vecs; i += step)
+      dtable[i] = z;
+    return;
+  }
+  const auto row_of = [&](int j) {
+    const long long id = ids[j];
+    return id >= 0 && id < V ? static_cast<int>(id) : EMB_NO_ROW;
+  };
+  const int lane = threadIdx.x & 31;
+  const int slice = lane >> 3;                         // which quarter of every group of 16 ids this thread compares with
+  const int i0 = blockIdx.x * EMB_RANK_TOKENS;
+  const int i = i0 + (threadIdx.x >> 5) * 8 + (lane & 7);
+  const int mine = i < T ? row_of(i) : 0;
+  int rank = 0;
+  for (int t0 = 0; t0 < T; t0 += EMB_RANK_TILE) {
+    const int n = T - t0 < EMB_RANK_TILE ? T - t0 : EMB_RANK_TILE;
+    __syncthreads();
+    for (int k = threadIdx.x; k < (n + 15) / 16 * 16; k += EW_THREADS)
+      tile[k] = k < n ? row_of(t0 + k) : 0x7fffffff;   // past the end: larger than any id
+    __syncthreads();
+    const int4* tv = reinterpret_cast<const int4*>(tile);
+    if (t0 + EMB_RANK_TILE <= i0 || t0 >= i0 + EMB_RANK_TOKENS) {
+      const int bound = mine + (t0 < i0 ? 1 : 0);      // ids before mine win ties, ids after it lose them
+#pragma unroll 4
+      for (int k = slice; k < (n + 15) / 16 * 4; k += 4) {
+        const int4 o = tv[k];
+        rank += (o.x < bound) + (o.y < bound) + (o.z < bound) + (o.w < bound);
+      }
+    } else {
+      for (int k = slice; k < (n + 15) / 16 * 4; k += 4) {
+        const int4 o = tv[k];
+        const int j = t0 + 4 * k;
+        rank += (o.x < mine + (j < i)) + (o.y < mine + (j + 1 < i)) + (o.z < mine + (j + 2 < i)) + (o.w < mine + (j + 3 < i));
+      }
+    }
+  }
+  rank += __shfl_xor_sync(0xffffffffu, rank, 8);
+  rank += __shfl_xor_sync(0xffffffffu, rank, 16);
+  if (slice == 0 && i < T) {
+    sorted_ids[rank] = mine;
+    perm[rank] = i;
+  }
+}
+
+// Step 2: a block sums EMB_CHUNK sorted tokens, whatever runs of equal ids they form: token frequencies follow a power
+// law, and a block per run left one block with hundreds of dependent row reads while the chip idled.  Eight row loads
+// are in flight at a time.  A run inside the chunk is written to its table row; the part of a run that reaches
+// over the chunk's start / end goes to part[chunk][0] / part[chunk][1] in fp32, and step 3 adds those up in order.
+// Measured, 8192 tokens by Zipf's law (the commonest id 480 times), N = 896: 10 us and 7 us for
+// step 3, against 292 us with a block per run.
+constexpr int EMB_CHUNK = 32;
+
 __global__ void __launch_bounds__(128)
-embedding_bwd_kernel(const long long* __restrict__ sorted_ids, const long long* __restrict__ perm,
-                     const bf16* __restrict__ dout, bf16* __restrict__ dtable, long long T, int N, long long V,
-                     int accumulate) {
-  const long long i = blockIdx.x;
-  const long long id = sorted_ids[i];
-  if (id < 0 || id >= V) return;
-  if (i > 0 && sorted_ids[i - 1] == id) return;
-  const int nvec = N / 8;
-  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-    float acc[8];
-    uint4* dst = reinterpret_cast<uint4*>(dtable + id * N) + v;
-    if (accumulate) unpack8(*dst, acc);
-    else
+embedding_bwd_kernel(const int* __restrict__ sorted_ids, const int* __restrict__ perm, const bf16* __restrict__ dout,
+                     bf16* __restrict__ dtable, float* __restrict__ part, int T, int N) {
+  __shared__ int sid[EMB_CHUNK + 2], src[EMB_CHUNK];   // sid[k + 1] = id of the chunk's k-th token, with both neighbours
+  const int r0 = blockIdx.x * EMB_CHUNK;
+  const int n = T - r0 < EMB_CHUNK ? T - r0 : EMB_CHUNK;
+  for (int k = threadIdx.x; k < EMB_CHUNK + 2; k += blockDim.x) {
+    const int r = r0 + k - 1;
+    sid[k] = r >= 0 && r < T ? sorted_ids[r] : -1;
+    if (k >= 1 && k <= n) src[k - 1] = perm[r];
+  }
+  __syncthreads();
+  const int v = blockIdx.y * blockDim.x + threadIdx.x;
+  if (v >= N / 8) return;
+  float acc[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    for (long long r = i; r < T && sorted_ids[r] == id; ++r) {
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  bool whole = sid[1] != sid[0];                       // the run being summed began inside this chunk
+  for (int k0 = 0; k0 < n; k0 += 8) {
+    uint4 u[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (k0 + q < n) u[q] = reinterpret_cast<const uint4*>(dout + static_cast<long long>(src[k0 + q]) * N)[v];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int k = k0 + q;
+      if (k >= n) break;
       float d[8];
-      unpack8(reinterpret_cast<const uint4*>(dout + perm[r] * N)[v], d);
+      unpack8(u[q], d);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] += d[j];
+      const bool ends = sid[k + 2] != sid[k + 1];      // also at the last token, whose neighbour is -1
+      if (ends || k + 1 == n) {
+        if (ends && whole) {
+          if (sid[k + 1] != EMB_NO_ROW) reinterpret_cast<uint4*>(dtable + static_cast<long long>(sid[k + 1]) * N)[v] = pack8(acc);
+        } else {
+          float4* o = reinterpret_cast<float4*>(part + (2LL * blockIdx.x + (whole ? 1 : 0)) * N) + 2 * v;
+          o[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+          o[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+        whole = true;
+      }
     }
-    *dst = pack8(acc);
   }
+}
+
+// Step 3: the block of the chunk in which a run begins that its last token does not end adds the parts of the chunks
+// that follow, in their order, and writes the row.
+__global__ void __launch_bounds__(128)
+embedding_bwd_span_kernel(const int* __restrict__ sorted_ids, bf16* __restrict__ dtable, const float* __restrict__ part, int T, int N) {
+  const int r0 = blockIdx.x * EMB_CHUNK, last = r0 + EMB_CHUNK - 1;
+  if (last + 1 >= T) return;
+  const int id = sorted_ids[last];
+  if (id == EMB_NO_ROW || sorted_ids[last + 1] != id) return;
+  if (r0 > 0 && sorted_ids[r0] == id && sorted_ids[r0 - 1] == id) return;     // began before this chunk
+  const int v = blockIdx.y * blockDim.x + threadIdx.x;
+  if (v >= N / 8) return;
+  int chunks = 0;                                      // chunks after this one that begin with the run
+  for (long long r = r0 + EMB_CHUNK; r < T && sorted_ids[r] == id; r += EMB_CHUNK) ++chunks;
+  const float4* p = reinterpret_cast<const float4*>(part) + 2 * v;
+  const long long ld = N / 4;                          // one part row in float4
+  const float4 a0 = p[(2LL * blockIdx.x + 1) * ld], b0 = p[(2LL * blockIdx.x + 1) * ld + 1];
+  float acc[8] = {a0.x, a0.y, a0.z, a0.w, b0.x, b0.y, b0.z, b0.w};
+#pragma unroll 4
+  for (int c = 1; c <= chunks; ++c) {
+    const float4 a = p[2LL * (blockIdx.x + c) * ld], b = p[2LL * (blockIdx.x + c) * ld + 1];
+    acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+    acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+  }
+  reinterpret_cast<uint4*>(dtable + static_cast<long long>(id) * N)[v] = pack8(acc);
 }
 
 // ------------------------------------------------------------------ cross-entropy on materialised logits
@@ -912,10 +1028,35 @@ int cb_embedding_fwd(const long long* ids, const void* table, void* out, long lo
   return static_cast<int>(cudaGetLastError());
 }
 
-int cb_embedding_bwd(const long long* sorted_ids, const long long* perm, const void* dout, void* dtable, long long T,
-                     int N, long long V, int accumulate, void* stream) {
-  if (N % 8 != 0 || T <= 0) return -1;
-  cb::embedding_bwd_kernel<<<static_cast<unsigned>(T), 128, 0, static_cast<cudaStream_t>(stream)>>>(sorted_ids, perm, static_cast<const cb::bf16*>(dout), static_cast<cb::bf16*>(dtable), T, N, V, accumulate);
+// Most tokens that cb_embedding_rank_fill sorts itself; more of them are sorted by the caller.
+int cb_embedding_rank_max() { return 32768; }
+
+// Zeroes dtable [V, N] and, with sorted_ids / perm given (T int32 each), sorts the T ids (stable).
+int cb_embedding_rank_fill(const long long* ids, int* sorted_ids, int* perm, void* dtable, long long T, int N, long long V,
+                           void* stream) {
+  if (N % 8 != 0 || T <= 0 || V <= 0 || V >= cb::EMB_NO_ROW) return -1;
+  if (sorted_ids != nullptr && T > cb_embedding_rank_max()) return -2;
+  const int rank_blocks = sorted_ids != nullptr ? static_cast<int>((T + cb::EMB_RANK_TOKENS - 1) / cb::EMB_RANK_TOKENS) : 0;
+  const long long vecs = V * (N / 8);
+  const int fill_blocks = grid_for(vecs, cb::EW_THREADS, 8);
+  cb::embedding_rank_fill_kernel<<<rank_blocks + fill_blocks, cb::EW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      ids, sorted_ids, perm, static_cast<int>(T), rank_blocks, static_cast<uint4*>(dtable), vecs, V);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// Rows of N floats that `part` of cb_embedding_bwd holds for T tokens.
+int cb_embedding_part_rows(long long T) { return static_cast<int>(2 * ((T + cb::EMB_CHUNK - 1) / cb::EMB_CHUNK)); }
+
+// dtable (zeroed) receives the sums of the rows of dout [T, N] over equal ids; sorted_ids ascending (ids that are no row
+// of the table hold 0x7ffffffe), perm the source token of each.
+int cb_embedding_bwd(const int* sorted_ids, const int* perm, const void* dout, void* dtable, float* part, long long T, int N,
+                     void* stream) {
+  if (N % 8 != 0 || T <= 0 || T > 0x7fffff00LL) return -1;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const dim3 grid(static_cast<unsigned>((T + cb::EMB_CHUNK - 1) / cb::EMB_CHUNK), (N / 8 + 127) / 128);
+  cb::embedding_bwd_kernel<<<grid, 128, 0, s>>>(sorted_ids, perm, static_cast<const cb::bf16*>(dout), static_cast<cb::bf16*>(dtable),
+                                                part, static_cast<int>(T), N);
+  cb::embedding_bwd_span_kernel<<<grid, 128, 0, s>>>(sorted_ids, static_cast<cb::bf16*>(dtable), part, static_cast<int>(T), N);
   return static_cast<int>(cudaGetLastError());
 }
 

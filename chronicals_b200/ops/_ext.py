@@ -44,7 +44,10 @@ _PROTOTYPES = {
     "cb_qk_rope": [P, P, P, P, P, L, I, I, I, L, L, I, I, L, P],
     "cb_debug_word": [P],
     "cb_embedding_fwd": [P, P, P, L, I, L, P],
-    "cb_embedding_bwd": [P, P, P, P, L, I, L, I, P],
+    "cb_embedding_rank_max": [],
+    "cb_embedding_part_rows": [L],
+    "cb_embedding_rank_fill": [P, P, P, P, L, I, L, P],
+    "cb_embedding_bwd": [P, P, P, P, P, L, I, P],
     "cb_ce_logits": [P, P, L, L, I, I, L, F, F, P, P, P],
     "cb_ce_logits_grad": [P, P, P, P, P, P, L, L, L, I, I, L, F, F, P],
     "cb_attn_fwd": [P, P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, P, P],
@@ -140,7 +143,7 @@ def lib() -> ctypes.CDLL:
 
 # device kernels launched by one call of each entry point (0: host-only query)
 _KERNELS_PER_CALL = {"cb_gemm2sm_supported": 0, "cb_gemm2sm_cost_milli": 0, "cb_cce_num_splits": 0, "cb_rmsnorm_max_n": 0, "cb_rmsnorm_bwd_blocks": 0, "cb_opt_chunk": 0,
-                     "cb_cce_combine": 2, "cb_rmsnorm_bwd": 2, "cb_grad_clip_coef": 2, "cb_attn_bwd": 3}
+                     "cb_embedding_rank_max": 0, "cb_embedding_part_rows": 0, "cb_embedding_bwd": 2, "cb_cce_combine": 2, "cb_rmsnorm_bwd": 2, "cb_grad_clip_coef": 2, "cb_attn_bwd": 3}
 LAUNCH_COUNT = [0]
 
 

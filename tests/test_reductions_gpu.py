@@ -46,3 +46,27 @@ def test_logits_cross_entropy_rows(rows, V, gap, shift, dtype):
     if gap:                                                       # nothing outside the rows was written
         assert torch.equal(buf[shift:].view(rows, V + gap)[:, :V], lg)
 
+
+# chunk and tile edges of the sort by counting, several tiles of ids, the range sorted by the library; one id only, ids
+# outside the table
+@pytest.mark.parametrize("T,V,N", [(1, 5, 8), (31, 40, 64), (32, 3, 896), (33, 1, 8), (64, 1000, 1032), (65, 7, 256),
+                                   (4097, 151, 896), (9000, 32000, 64), (33000, 500, 64)])
+def test_embedding_backward_runs(T, V, N):
+    g = _gen(T + V)
+    table = torch.randn(V, N, device=DEV, generator=g).to(torch.bfloat16).requires_grad_()
+    ids = (torch.exp(torch.rand(T, device=DEV, generator=g) * math.log(V + 1)) - 1).long().clamp_(0, V - 1)
+    if T > 64:
+        ids[40:60], ids[62] = V + 5, -1                           # read row 0 forward, take no part backward
+    dy = torch.randn(T, N, device=DEV, generator=g).to(torch.bfloat16)
+    y = ops.embedding(ids, table)
+    y.backward(dy)
+    ok = (ids >= 0) & (ids < V)
+    assert torch.equal(y, table.detach()[torch.where(ok, ids, torch.zeros_like(ids))])
+    want = torch.zeros(V, N, dtype=torch.float64, device=DEV).index_add_(0, ids[ok], dy[ok].double())
+    size = torch.zeros(V, N, dtype=torch.float64, device=DEV).index_add_(0, ids[ok], dy[ok].double().abs())
+    # one rounding to bf16, and T fp32 additions of at most `size`
+    assert ((table.grad.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -23 * 40 * size).all()
+    first = table.grad.clone()
+    table.grad = None
+    ops.embedding(ids, table).backward(dy)
+    assert torch.equal(first, table.grad)

@@ -49,83 +49,101 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return u;
 }
 
-// Sum over the TPR threads that share one row.  TPR == 32: shuffle only.  Otherwise the
-// group's warps exchange through shared memory; every thread of the block must call it.
-template <int TPR>
-__device__ __forceinline__ float group_sum(float v, float* sred) {
+// 16 bytes from global to this thread's own place in shared memory, without passing through registers.  A thread reads
+// only what it copied itself, so a ring of such places needs no barrier: its own wait is enough.
+__device__ __forceinline__ void cp_async16(uint4* dst, const uint4* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// How rows are laid over threads.  Up to 1024 columns a warp takes a row (shuffles only, eight rows a block); wider rows
+// take a block that is just wide enough for two vectors of 8 a thread, and four beyond 5120 columns.
+template <int VPL, bool WARP_ROW>
+struct RowLayout {
+  int t, tpr, group, groups;
+  __device__ __forceinline__ RowLayout() {
+    t = WARP_ROW ? static_cast<int>(threadIdx.x & 31) : static_cast<int>(threadIdx.x);
+    tpr = WARP_ROW ? 32 : static_cast<int>(blockDim.x);
+    group = WARP_ROW ? static_cast<int>(threadIdx.x >> 5) : 0;
+    groups = WARP_ROW ? static_cast<int>(blockDim.x >> 5) : 1;
+  }
+};
+
+// Sum over the threads of one row.  `sred` has two halves of 32 floats used in turn (`flip`), so that one barrier a row
+// is enough: nobody writes a half again before everybody has left the barrier after reading it.
+template <bool WARP_ROW>
+__device__ __forceinline__ float row_sum(float v, float* sred, int flip) {
   v = warp_sum(v);
-  if (TPR == 32) return v;
-  const int warp = threadIdx.x >> 5;
-  constexpr int WPG = TPR / 32;
-  if ((threadIdx.x & 31) == 0) sred[warp] = v;
+  if (WARP_ROW) return v;
+  float* half = sred + 32 * flip;
+  if ((threadIdx.x & 31) == 0) half[threadIdx.x >> 5] = v;
   __syncthreads();
-  const int g0 = (warp / WPG) * WPG;
+  const int nw = static_cast<int>(blockDim.x >> 5);
   float t = 0.f;
-#pragma unroll
-  for (int i = 0; i < WPG; ++i) t += sred[g0 + i];
-  __syncthreads();
+  for (int i = 0; i < nw; ++i) t += half[i];
   return t;
 }
 
 // ------------------------------------------------------------------ RMSNorm forward
 // h = x (+ res);  y = h * rsqrt(mean(h^2) + eps) * (w + offset);  rstd saved.
-// N % 8 == 0, N <= 8 * TPR * VPL.
-template <int TPR, int VPL>
-__global__ void __launch_bounds__(EW_THREADS)
+// N % 8 == 0, N <= 8 * VPL * (threads of a row).
+template <int VPL, bool WARP_ROW>
+__global__ void __launch_bounds__(WARP_ROW ? EW_THREADS : 320)
 rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, const bf16* __restrict__ w,
                    bf16* __restrict__ y, bf16* __restrict__ h_out, float* __restrict__ rstd_out, int M, int N,
                    float eps, float offset) {
-  __shared__ float sred[EW_THREADS / 32];
-  constexpr int RPB = EW_THREADS / TPR;
-  const int group = threadIdx.x / TPR;
-  const int t = threadIdx.x % TPR;
+  __shared__ float sred[64];
+  const RowLayout<VPL, WARP_ROW> L;
   const int nvec = N / 8;
-  for (int base = blockIdx.x * RPB; base < M; base += gridDim.x * RPB) {
-    const int row = base + group;
-    const bool active = row < M;
-    float h[VPL][8];
+  const int step = gridDim.x * L.groups;
+  int flip = 0;
+  for (long long row = blockIdx.x * L.groups + L.group; row < M; row += step) {
+    const uint4* xp = reinterpret_cast<const uint4*>(x + row * N);
+    const uint4* rp = res ? reinterpret_cast<const uint4*>(res + row * N) : nullptr;
+    uint4* hp = h_out ? reinterpret_cast<uint4*>(h_out + row * N) : nullptr;
+    uint4 hr[VPL];
     float ss = 0.f;
-    if (active) {
-      const uint4* xp = reinterpret_cast<const uint4*>(x + static_cast<long long>(row) * N);
-      const uint4* rp = res ? reinterpret_cast<const uint4*>(res + static_cast<long long>(row) * N) : nullptr;
-      uint4* hp = h_out ? reinterpret_cast<uint4*>(h_out + static_cast<long long>(row) * N) : nullptr;
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int v = t + i * TPR;
-        if (v < nvec) {
-          unpack8(xp[v], h[i]);
-          if (rp) {
-            float r[8];
-            unpack8(rp[v], r);
+    for (int i = 0; i < VPL; ++i)
+      if (L.t + i * L.tpr < nvec) hr[i] = xp[L.t + i * L.tpr];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) h[i][j] += r[j];
-            const uint4 hb = pack8(h[i]);   // the sum is stored in bf16; normalise what is stored
-            if (hp) hp[v] = hb;
-            unpack8(hb, h[i]);
-          }
+    for (int i = 0; i < VPL; ++i) {
+      const int v = L.t + i * L.tpr;
+      if (v < nvec) {
+        float f[8];
+        unpack8(hr[i], f);
+        if (rp) {
+          float r[8];
+          unpack8(rp[v], r);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) ss += h[i][j] * h[i][j];
+          for (int j = 0; j < 8; ++j) f[j] += r[j];
+          hr[i] = pack8(f);                          // the sum is stored in bf16; normalise what is stored
+          if (hp) hp[v] = hr[i];
+          unpack8(hr[i], f);
         }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
       }
     }
-    ss = group_sum<TPR>(ss, sred);
-    if (active) {
-      const float rstd = rsqrtf(ss / static_cast<float>(N) + eps);
-      if (t == 0 && rstd_out) rstd_out[row] = rstd;
-      const uint4* wp = reinterpret_cast<const uint4*>(w);
-      uint4* yp = reinterpret_cast<uint4*>(y + static_cast<long long>(row) * N);
+    ss = row_sum<WARP_ROW>(ss, sred, flip);
+    const float rstd = rsqrtf(ss / static_cast<float>(N) + eps);
+    if (L.t == 0 && rstd_out) rstd_out[row] = rstd;
+    uint4* yp = reinterpret_cast<uint4*>(y + row * N);
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int v = t + i * TPR;
-        if (v < nvec) {
-          float wf[8], o[8];
-          unpack8(wp[v], wf);
+    for (int i = 0; i < VPL; ++i) {
+      const int v = L.t + i * L.tpr;
+      if (v < nvec) {
+        float f[8], wf[8], o[8];
+        unpack8(hr[i], f);
+        unpack8(reinterpret_cast<const uint4*>(w)[v], wf);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = h[i][j] * rstd * (wf[j] + offset);
-          yp[v] = pack8(o);
-        }
+        for (int j = 0; j < 8; ++j) o[j] = f[j] * rstd * (wf[j] + offset);
+        yp[v] = pack8(o);
       }
     }
+    flip ^= 1;
   }
 }
 
@@ -133,115 +151,127 @@ rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, con
 // xhat = h*rstd; g = dy*(w+offset); dx = rstd*(g - xhat*mean(g*xhat)) (+ dres_in);
 // dw[n] = sum_rows dy*xhat, accumulated per block in registers and written as one
 // [gridDim.x, N] fp32 partial (reduced by rmsnorm_dw_reduce_kernel).
-template <int TPR, int VPL>
-__global__ void __launch_bounds__(EW_THREADS, 2)
+// Bound by memory (four tensors).  The sums of dw keep two blocks an SM at most, and with the loads of a row waiting
+// behind the reduction and the stores of the one before, they kept memory busy two thirds of the time; now each thread
+// has its vectors of the next RING - 1 rows in flight through the ring.  Measured: 16,384 x 5120 144 -> 109 us
+// (6.1 TB/s), 16,384 x 2048 68 -> 49, 32,768 x 896 50 -> 43, 8192 x 896 16.3 -> 16.0.  The forward kernel has enough
+// blocks an SM without a ring (16,384 x 5120: 66 us with one, 58 without).
+// Dynamic shared memory: RING * (dres_in ? 3 : 2) * VPL * blockDim.x vectors, and no less than [groups, N] floats.
+template <int VPL, bool WARP_ROW, int RING>
+__global__ void __launch_bounds__(WARP_ROW ? EW_THREADS : 320, 2)
 rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ h, const bf16* __restrict__ w,
                    const float* __restrict__ rstd_in, const bf16* __restrict__ dres_in, bf16* __restrict__ dx,
                    float* __restrict__ dw_part, int M, int N, float offset) {
-  __shared__ float sred[EW_THREADS / 32];
-  extern __shared__ float sdw[];  // [RPB, N] per-group accumulators, used when several row groups share a block
-  constexpr int RPB = EW_THREADS / TPR;
-  const int group = threadIdx.x / TPR;
-  const int t = threadIdx.x % TPR;
+  extern __shared__ __align__(16) uint4 ring[];
+  __shared__ float sred[64];
+  const RowLayout<VPL, WARP_ROW> L;
   const int nvec = N / 8;
+  const int step = gridDim.x * L.groups;
+  const int row0 = blockIdx.x * L.groups + L.group;
+  const int inputs = dres_in ? 3 : 2;
+  const auto slot = [&](int stage, int in, int i) { return ring + ((stage * inputs + in) * VPL + i) * blockDim.x + threadIdx.x; };
+  const auto fetch = [&](long long row, int stage) {
+    if (row < M) {
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        const int v = L.t + i * L.tpr;
+        if (v < nvec) {
+          cp_async16(slot(stage, 0, i), reinterpret_cast<const uint4*>(dy + row * N) + v);
+          cp_async16(slot(stage, 1, i), reinterpret_cast<const uint4*>(h + row * N) + v);
+          if (dres_in) cp_async16(slot(stage, 2, i), reinterpret_cast<const uint4*>(dres_in + row * N) + v);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  uint4 wr[VPL];
   float dwacc[VPL][8];
 #pragma unroll
-  for (int i = 0; i < VPL; ++i)
+  for (int i = 0; i < VPL; ++i) {
+    if (L.t + i * L.tpr < nvec) wr[i] = reinterpret_cast<const uint4*>(w)[L.t + i * L.tpr];
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
-
-  for (int base = blockIdx.x * RPB; base < M; base += gridDim.x * RPB) {
-    const int row = base + group;
-    const bool active = row < M;
-    // One memory round trip per row: dy, h and the pass-through gradient are all requested before anything is
-    // consumed, and stay packed (bf16) in registers until the second pass converts them again.
-    uint4 dyr[VPL], hr[VPL], rr[VPL];
-    float dot = 0.f;
-    float rstd = 0.f;
-    const uint4* wp = reinterpret_cast<const uint4*>(w);
-    if (active) {
-      rstd = rstd_in[row];
-      const uint4* dyp = reinterpret_cast<const uint4*>(dy + static_cast<long long>(row) * N);
-      const uint4* hp = reinterpret_cast<const uint4*>(h + static_cast<long long>(row) * N);
-      const uint4* rp = dres_in ? reinterpret_cast<const uint4*>(dres_in + static_cast<long long>(row) * N) : nullptr;
-#pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int v = t + i * TPR;
-        if (v < nvec) {
-          dyr[i] = dyp[v];
-          hr[i] = hp[v];
-          if (rp) rr[i] = rp[v];
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int v = t + i * TPR;
-        if (v < nvec) {
-          float d[8], x[8], wf[8];
-          unpack8(dyr[i], d);
-          unpack8(hr[i], x);
-          unpack8(wp[v], wf);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float xh = x[j] * rstd;
-            dot += d[j] * (wf[j] + offset) * xh;
-            dwacc[i][j] += d[j] * xh;
-          }
-        }
-      }
-    }
-    dot = group_sum<TPR>(dot, sred);
-    if (active) {
-      const float mean = dot / static_cast<float>(N);
-      uint4* dxp = reinterpret_cast<uint4*>(dx + static_cast<long long>(row) * N);
-#pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int v = t + i * TPR;
-        if (v < nvec) {
-          float d[8], x[8], wf[8], o[8];
-          unpack8(dyr[i], d);
-          unpack8(hr[i], x);
-          unpack8(wp[v], wf);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = rstd * (d[j] * (wf[j] + offset) - x[j] * rstd * mean);
-          if (dres_in) {
-            float r[8];
-            unpack8(rr[i], r);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += r[j];
-          }
-          dxp[v] = pack8(o);
-        }
-      }
-    }
   }
-  // block-level reduction of dw over the row groups, then one partial row per block: every group parks its
-  // accumulators in its own [N] row of shared memory and the block sums the RPB rows column by column
-  // (fixed order, no atomics)
-  if (RPB > 1) {
-    float* mine = sdw + static_cast<size_t>(group) * N;
+  for (int k = 0; k < RING - 1; ++k) fetch(row0 + static_cast<long long>(k) * step, k);
+  float rstd_next = row0 < M ? rstd_in[row0] : 0.f;
+  int stage = 0, flip = 0;
+  for (long long row = row0; row < M; row += step) {
+    const float rstd = rstd_next;
+    if (row + step < M) rstd_next = rstd_in[row + step];
+    fetch(row + static_cast<long long>(RING - 1) * step, stage == 0 ? RING - 1 : stage - 1);
+    cp_async_wait<RING - 1>();
+    float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-      const int v = t + i * TPR;
+      if (L.t + i * L.tpr < nvec) {
+        float d[8], x[8], wf[8];
+        unpack8(*slot(stage, 0, i), d);
+        unpack8(*slot(stage, 1, i), x);
+        unpack8(wr[i], wf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xh = x[j] * rstd;
+          dot += d[j] * (wf[j] + offset) * xh;
+          dwacc[i][j] += d[j] * xh;
+        }
+      }
+    }
+    dot = row_sum<WARP_ROW>(dot, sred, flip);
+    const float mean = dot / static_cast<float>(N);
+    uint4* dxp = reinterpret_cast<uint4*>(dx + row * N);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      const int v = L.t + i * L.tpr;
       if (v < nvec) {
-        reinterpret_cast<float4*>(mine + v * 8)[0] = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
-        reinterpret_cast<float4*>(mine + v * 8)[1] = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
+        float d[8], x[8], wf[8], o[8];
+        unpack8(*slot(stage, 0, i), d);
+        unpack8(*slot(stage, 1, i), x);
+        unpack8(wr[i], wf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = rstd * (d[j] * (wf[j] + offset) - x[j] * rstd * mean);
+        if (dres_in) {
+          float r[8];
+          unpack8(*slot(stage, 2, i), r);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] += r[j];
+        }
+        dxp[v] = pack8(o);
+      }
+    }
+    stage = stage + 1 == RING ? 0 : stage + 1;
+    flip ^= 1;
+  }
+  // one partial row of dw per block: with several rows in a block every group parks its sums in its own [N] row of
+  // shared memory (the ring is done with) and the block adds them column by column (fixed order, no atomics)
+  float* out = dw_part + static_cast<long long>(blockIdx.x) * N;
+  if (WARP_ROW) {
+    float* sdw = reinterpret_cast<float*>(ring);
+    cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      const int v = L.t + i * L.tpr;
+      if (v < nvec) {
+        float4* m = reinterpret_cast<float4*>(sdw + static_cast<size_t>(L.group) * N) + 2 * v;
+        m[0] = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
+        m[1] = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
       }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < N; i += EW_THREADS) {
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
       float a = 0.f;
 #pragma unroll
-      for (int r = 0; r < RPB; ++r) a += sdw[static_cast<size_t>(r) * N + i];
-      dw_part[static_cast<long long>(blockIdx.x) * N + i] = a;
+      for (int r = 0; r < EW_THREADS / 32; ++r) a += sdw[static_cast<size_t>(r) * N + i];
+      out[i] = a;
     }
   } else {
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-      const int v = t + i * TPR;
-      if (v < nvec)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) dw_part[static_cast<long long>(blockIdx.x) * N + v * 8 + j] = dwacc[i][j];
+      const int v = L.t + i * L.tpr;
+      if (v < nvec) {
+        reinterpret_cast<float4*>(out)[2 * v] = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
+        reinterpret_cast<float4*>(out)[2 * v + 1] = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
+      }
     }
   }
 }
@@ -280,24 +310,23 @@ colsum_partial_kernel(const bf16* __restrict__ x, long long ld, long long M, int
   reinterpret_cast<float4*>(o)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
 }
 
-// 256 threads = 32 columns x 8 row slices; each slice sums every 8th partial row, then the slices combine
-__global__ void rmsnorm_dw_reduce_kernel(const float* __restrict__ part, int nblocks, int N, bf16* __restrict__ dw,
-                                         int accumulate) {
-  __shared__ float red[8][33];
+// 1024 threads = 32 columns x 32 row slices; each slice sums every 32nd partial row, then the slices combine.  The
+// partials lie in L2 and the sum is bound by latency: with 32 slices (8 before) a thread waits for a quarter of the loads.
+__global__ void __launch_bounds__(1024)
+rmsnorm_dw_reduce_kernel(const float* __restrict__ part, int nblocks, int N, bf16* __restrict__ dw, int accumulate) {
+  __shared__ float red[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int n = blockIdx.x * 32 + tx;
   float s = 0.f;
-  if (n < N)
-    for (int b = ty; b < nblocks; b += 8) s += part[static_cast<long long>(b) * N + n];
+  if (n < N) {
+#pragma unroll 4
+    for (int b = ty; b < nblocks; b += 32) s += part[static_cast<long long>(b) * N + n];
+  }
   red[ty][tx] = s;
   __syncthreads();
-  if (ty == 0 && n < N) {
-    float t = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t += red[i][tx];
-    if (accumulate) t += __bfloat162float(dw[n]);
-    dw[n] = __float2bfloat16(t);
-  }
+  const float t = warp_sum(red[tx][ty]);               // warp ty adds the slices of column ty
+  const int m = blockIdx.x * 32 + ty;
+  if (tx == 0 && m < N) dw[m] = __float2bfloat16(accumulate ? t + __bfloat162float(dw[m]) : t);
 }
 
 // ------------------------------------------------------------------ gated activations
@@ -886,13 +915,42 @@ int ce_split(long long rows, int V) {
   while (split < 8 && rows * split < 4LL * sm_count() && V / (2 * split) >= 4096) split *= 2;
   return split;
 }
-// rows-per-thread-group choice: the smallest group whose registers hold the row (VPL = 4 vectors of 8)
-int pick_tpr(int N) {
+// Layout of a row of N columns (see RowLayout): vectors a thread, threads a block, rows a block; vpl = 0: too wide
+struct RowPlan {
+  int vpl, threads, rows;
+};
+RowPlan row_plan(int N) {
   const int nvec = N / 8;
-  if (nvec <= 32 * 4) return 32;
-  if (nvec <= 128 * 4) return 128;
-  if (nvec <= 256 * 4) return 256;
-  return 0;
+  if (nvec <= 32 * 4) return {4, cb::EW_THREADS, cb::EW_THREADS / 32};
+  if (nvec <= 640) return {2, (nvec + 63) / 64 * 32, 1};
+  if (nvec <= 256 * 4) return {4, (nvec + 127) / 128 * 32, 1};
+  return {0, 0, 0};
+}
+constexpr int RMS_BWD_RING2 = 3, RMS_BWD_RING4 = 2;   // ring depth by vectors a thread
+
+template <typename K>
+int rms_smem(K kern, size_t bytes) {
+  if (bytes <= 40 * 1024) return 0;                    // with the kernels' static arrays within the default 48 KB
+  return static_cast<int>(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+}
+
+int launch_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const void* dres_in, void* dx,
+                       float* part, int M, int N, float offset, int grid, cudaStream_t s) {
+  const RowPlan pl = row_plan(N);
+  const int ring = pl.vpl == 2 ? RMS_BWD_RING2 : RMS_BWD_RING4;
+  size_t smem = static_cast<size_t>(ring) * (dres_in ? 3 : 2) * pl.vpl * pl.threads * 16;
+  if (pl.rows > 1) smem = std::max(smem, static_cast<size_t>(pl.rows) * N * sizeof(float));
+  const auto go = [&](auto kern) {
+    const int e = rms_smem(kern, smem);
+    if (e) return e;
+    kern<<<grid, pl.threads, smem, s>>>(static_cast<const cb::bf16*>(dy), static_cast<const cb::bf16*>(h),
+                                        static_cast<const cb::bf16*>(w), rstd, static_cast<const cb::bf16*>(dres_in),
+                                        static_cast<cb::bf16*>(dx), part, M, N, offset);
+    return static_cast<int>(cudaGetLastError());
+  };
+  if (pl.rows > 1) return go(cb::rmsnorm_bwd_kernel<4, true, RMS_BWD_RING4>);
+  if (pl.vpl == 2) return go(cb::rmsnorm_bwd_kernel<2, false, RMS_BWD_RING2>);
+  return go(cb::rmsnorm_bwd_kernel<4, false, RMS_BWD_RING4>);
 }
 }  // namespace
 
@@ -917,48 +975,43 @@ int cb_debug_word(long long* out2) {
 }
 
 int cb_rmsnorm_bwd_blocks(int M, int N) {
-  const int tpr = pick_tpr(N);
-  if (tpr == 0) return 0;
-  return grid_for(M, cb::EW_THREADS / tpr, 2);
+  const RowPlan pl = row_plan(N);
+  if (pl.vpl == 0) return 0;
+  // as many blocks as an SM's shared memory holds (16,384 x 5120: 145 us with one, 109 with two, 120 in a wave and a
+  // half): two of 256 threads with four vectors each, else as many as make 672 threads
+  const int per_sm = pl.vpl == 4 ? 2 : std::min(6, 672 / pl.threads);
+  return grid_for(M, pl.rows, per_sm);
 }
 
 int cb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd, int M, int N,
                    float eps, float offset, void* stream) {
   if (N % 8 != 0) return -1;
-  const int tpr = pick_tpr(N);
-  if (tpr == 0) return -2;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const cb::bf16* xp = static_cast<const cb::bf16*>(x);
-  const cb::bf16* rp = static_cast<const cb::bf16*>(res);
-  const cb::bf16* wp = static_cast<const cb::bf16*>(w);
-  cb::bf16* yp = static_cast<cb::bf16*>(y);
-  cb::bf16* hp = static_cast<cb::bf16*>(h_out);
-  const int grid = grid_for(M, cb::EW_THREADS / tpr, 8);
-  if (tpr == 32) cb::rmsnorm_fwd_kernel<32, 4><<<grid, cb::EW_THREADS, 0, s>>>(xp, rp, wp, yp, hp, rstd, M, N, eps, offset);
-  else if (tpr == 128) cb::rmsnorm_fwd_kernel<128, 4><<<grid, cb::EW_THREADS, 0, s>>>(xp, rp, wp, yp, hp, rstd, M, N, eps, offset);
-  else cb::rmsnorm_fwd_kernel<256, 4><<<grid, cb::EW_THREADS, 0, s>>>(xp, rp, wp, yp, hp, rstd, M, N, eps, offset);
-  return static_cast<int>(cudaGetLastError());
+  const RowPlan pl = row_plan(N);
+  if (pl.vpl == 0) return -2;
+  // enough short blocks that the last ones even out (16,384 x 5120: 65 us with 8 an SM, 58 with 16, 60 with one a row)
+  const int grid = grid_for(M, pl.rows, 16);
+  const auto go = [&](auto kern) {
+    kern<<<grid, pl.threads, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const cb::bf16*>(x), static_cast<const cb::bf16*>(res), static_cast<const cb::bf16*>(w),
+        static_cast<cb::bf16*>(y), static_cast<cb::bf16*>(h_out), rstd, M, N, eps, offset);
+    return static_cast<int>(cudaGetLastError());
+  };
+  if (pl.rows > 1) return go(cb::rmsnorm_fwd_kernel<4, true>);
+  if (pl.vpl == 2) return go(cb::rmsnorm_fwd_kernel<2, false>);
+  return go(cb::rmsnorm_fwd_kernel<4, false>);
 }
 
 // dw_part: scratch of cb_rmsnorm_bwd_blocks(M, N) * N floats.
 int cb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const void* dres_in, void* dx,
                    void* dw, float* dw_part, int M, int N, float offset, int accumulate_dw, void* stream) {
   if (N % 8 != 0) return -1;
-  const int tpr = pick_tpr(N);
-  if (tpr == 0) return -2;
+  if (row_plan(N).vpl == 0) return -2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const cb::bf16* dyp = static_cast<const cb::bf16*>(dy);
-  const cb::bf16* hp = static_cast<const cb::bf16*>(h);
-  const cb::bf16* wp = static_cast<const cb::bf16*>(w);
-  const cb::bf16* rp = static_cast<const cb::bf16*>(dres_in);
-  cb::bf16* dxp = static_cast<cb::bf16*>(dx);
   const int grid = cb_rmsnorm_bwd_blocks(M, N);
-  const size_t smem = tpr == 256 ? 0 : static_cast<size_t>(cb::EW_THREADS / tpr) * N * sizeof(float);   // <= 32 KB
-  if (tpr == 32) cb::rmsnorm_bwd_kernel<32, 4><<<grid, cb::EW_THREADS, smem, s>>>(dyp, hp, wp, rstd, rp, dxp, dw_part, M, N, offset);
-  else if (tpr == 128) cb::rmsnorm_bwd_kernel<128, 4><<<grid, cb::EW_THREADS, smem, s>>>(dyp, hp, wp, rstd, rp, dxp, dw_part, M, N, offset);
-  else cb::rmsnorm_bwd_kernel<256, 4><<<grid, cb::EW_THREADS, smem, s>>>(dyp, hp, wp, rstd, rp, dxp, dw_part, M, N, offset);
+  const int e = launch_rmsnorm_bwd(dy, h, w, rstd, dres_in, dx, dw_part, M, N, offset, grid, s);
+  if (e) return e;
   if (dw != nullptr)
-    cb::rmsnorm_dw_reduce_kernel<<<(N + 31) / 32, 256, 0, s>>>(dw_part, grid, N, static_cast<cb::bf16*>(dw), accumulate_dw);
+    cb::rmsnorm_dw_reduce_kernel<<<(N + 31) / 32, 1024, 0, s>>>(dw_part, grid, N, static_cast<cb::bf16*>(dw), accumulate_dw);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -978,7 +1031,7 @@ int cb_colsum_bf16(const void* x, void* out, float* part, long long M, int N, lo
   const int nvec = N / 8;
   dim3 grid(blocks, (nvec + cb::EW_THREADS - 1) / cb::EW_THREADS);
   cb::colsum_partial_kernel<<<grid, cb::EW_THREADS, 0, s>>>(static_cast<const cb::bf16*>(x), ld, M, N, part);
-  cb::rmsnorm_dw_reduce_kernel<<<(N + 31) / 32, 256, 0, s>>>(part, blocks, N, static_cast<cb::bf16*>(out), 0);
+  cb::rmsnorm_dw_reduce_kernel<<<(N + 31) / 32, 1024, 0, s>>>(part, blocks, N, static_cast<cb::bf16*>(out), 0);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1189,27 +1242,20 @@ int cb_rmsnorm_bwd_noalloc(const void* dy, const void* h, const void* w, const f
                            void* dx, void* dw, int M, int N, float offset, int accumulate_dw, void* stream) {
   if (M <= 0 || N <= 0 || N % 8 != 0) return -1;
   if (N > NOALLOC_MAX_N) return -2;                     // beyond the built-in scratch: use cb_rmsnorm_bwd
-  const int tpr = pick_tpr(N);
-  if (tpr == 0) return -2;
+  const RowPlan pl = row_plan(N);
+  if (pl.vpl == 0) return -2;
   float* part = nullptr;
   const int rc = noalloc_scratch(&part);
   if (rc != 0) return rc;
-  int grid = grid_for(M, cb::EW_THREADS / tpr, 1);
+  int grid = grid_for(M, pl.rows, 1);
   if (grid > NOALLOC_MAX_BLOCKS) grid = NOALLOC_MAX_BLOCKS;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const cb::bf16* dyp = static_cast<const cb::bf16*>(dy);
-  const cb::bf16* hp = static_cast<const cb::bf16*>(h);
-  const cb::bf16* wp = static_cast<const cb::bf16*>(w);
-  const cb::bf16* rp = static_cast<const cb::bf16*>(dres_in);
-  cb::bf16* dxp = static_cast<cb::bf16*>(dx);
-  const size_t smem = tpr == 256 ? 0 : static_cast<size_t>(cb::EW_THREADS / tpr) * N * sizeof(float);
   // every block writes all N entries of its own partial row before the reduction reads them, so
   // nothing left in the array by an earlier call can leak into this one
-  if (tpr == 32) cb::rmsnorm_bwd_kernel<32, 4><<<grid, cb::EW_THREADS, smem, s>>>(dyp, hp, wp, rstd, rp, dxp, part, M, N, offset);
-  else if (tpr == 128) cb::rmsnorm_bwd_kernel<128, 4><<<grid, cb::EW_THREADS, smem, s>>>(dyp, hp, wp, rstd, rp, dxp, part, M, N, offset);
-  else cb::rmsnorm_bwd_kernel<256, 4><<<grid, cb::EW_THREADS, smem, s>>>(dyp, hp, wp, rstd, rp, dxp, part, M, N, offset);
+  const int e = launch_rmsnorm_bwd(dy, h, w, rstd, dres_in, dx, part, M, N, offset, grid, s);
+  if (e) return e;
   if (dw != nullptr)
-    cb::rmsnorm_dw_reduce_kernel<<<(N + 31) / 32, 256, 0, s>>>(part, grid, N, static_cast<cb::bf16*>(dw), accumulate_dw);
+    cb::rmsnorm_dw_reduce_kernel<<<(N + 31) / 32, 1024, 0, s>>>(part, grid, N, static_cast<cb::bf16*>(dw), accumulate_dw);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -70,3 +70,29 @@ def test_embedding_backward_runs(T, V, N):
     table.grad = None
     ops.embedding(ids, table).backward(dy)
     assert torch.equal(first, table.grad)
+
+
+# one vector, a warp's row at its widest, the narrowest and the widest block with two vectors a thread (with a ragged last
+# vector), the first and the last width with four; fewer rows than the ring, rows that wrap it, more rows than blocks
+@pytest.mark.parametrize("M,N", [(1, 8), (3, 1024), (5, 1032), (700, 2056), (2, 5120), (301, 5120), (1, 5128), (613, 6664), (299, 8192),
+                                 (5000, 264)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_rmsnorm_layouts(M, N, residual):
+    g = _gen(M + N)
+    x, dy, dh = (torch.randn(M, N, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3))
+    w = (1 + 0.1 * torch.randn(N, device=DEV, generator=g)).to(torch.bfloat16)
+    xr, wr = x.double().requires_grad_(), w.double().requires_grad_()
+    yr = xr * torch.rsqrt(xr.square().mean(-1, keepdim=True) + 1e-6) * wr
+    x.requires_grad_(), w.requires_grad_()
+    if residual:
+        y, h = ops.rmsnorm_residual(x, w)
+        torch.autograd.backward((y, h), (dy, dh))
+        torch.autograd.backward((yr, xr * 1.0), (dy.double(), dh.double()))
+    else:
+        y = ops.rmsnorm(x, w)
+        y.backward(dy)
+        yr.backward(dy.double())
+    size = (dy.double() * yr.detach()).abs().sum(0)               # of the terms that a column of dw adds up
+    for got, want, slack in ((y, yr, 1e-5), (x.grad, xr.grad, 2e-5), (w.grad, wr.grad, 1e-5 * size + 1e-5)):
+        # one rounding to bf16 and fp32 sums (dx of a residual cancels: its terms are of order one)
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()

@@ -1537,7 +1537,16 @@ int cb_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
   }
   // scratch_is_zero: the caller keeps dq_acc / dk_part / dv_part between calls; they arrive all zero and the finalize
   // kernel leaves them all zero again, so the three clears are skipped
-  if (!scratch_is_zero) CB_CHECK_CUDA(cudaMemsetAsync(dq_acc, 0, sizeof(float) * static_cast<size_t>(T) * hq * D, s));
+  if (!scratch_is_zero) {
+    // one clear where the three accumulators follow each other
+    const size_t nq = static_cast<size_t>(T) * hq * D, nk = static_cast<size_t>(T) * hk * D;
+    const bool joined = dk_part == dq_acc + nq && dv_part == dk_part + nk;
+    CB_CHECK_CUDA(cudaMemsetAsync(dq_acc, 0, sizeof(float) * (joined ? nq + 2 * nk : nq), s));
+    if (!joined) {
+      CB_CHECK_CUDA(cudaMemsetAsync(dk_part, 0, sizeof(float) * nk, s));
+      CB_CHECK_CUDA(cudaMemsetAsync(dv_part, 0, sizeof(float) * nk, s));
+    }
+  }
   cb::AttnArgs a = {};
   a.T = T; a.hq = hq; a.hk = hk; a.n_docs = n_docs; a.cu = cu; a.scale = scale;
   a.lse = const_cast<float*>(lse); a.delta = delta; a.dq_acc = dq_acc; a.dk_part = dk_part; a.dv_part = dv_part;
@@ -1546,10 +1555,6 @@ int cb_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
   // Two threads per score row, S / dP / dQ sharing TMEM columns, dK / dV accumulated per kv head with red.add
   // (so those buffers start from zero).  D = 64 additionally fits two CTAs per SM.
   const int part_heads = hk;
-  if (!scratch_is_zero) {
-    CB_CHECK_CUDA(cudaMemsetAsync(dk_part, 0, sizeof(float) * static_cast<size_t>(T) * hk * D, s));
-    CB_CHECK_CUDA(cudaMemsetAsync(dv_part, 0, sizeof(float) * static_cast<size_t>(T) * hk * D, s));
-  }
   if (D == 64) {
     static bool cfg = false;
     if (!cfg) { e = set_smem(cb::attn_bwd2_kernel<64>, cb::Bwd2Smem<64>::TOTAL); if (e) return e; cfg = true; }

@@ -80,17 +80,19 @@ __device__ unsigned long long cb_attn_phase[2][16];
 __device__ __forceinline__ bool locate_tile(const int* cu, int n_docs, int b, int& start, int& len, int& weight, int& nblk,
                                             int* beyond = nullptr) {
   const int lane = threadIdx.x & 31;
-  int maxnb = 0;
-  for (int d = lane; d < n_docs; d += 32) maxnb = max(maxnb, (cu[d + 1] - cu[d] + 127) >> 7);
+  // the blocks of the first 32 documents stay in a register (their lookup per level was most of the search's time)
+  const int nb0 = lane < n_docs ? (cu[lane + 1] - cu[lane] + 127) >> 7 : 0;
+  int maxnb = nb0;
+  for (int d = lane + 32; d < n_docs; d += 32) maxnb = max(maxnb, (cu[d + 1] - cu[d] + 127) >> 7);
   maxnb = __reduce_max_sync(0xffffffffu, maxnb);
   for (int L = maxnb; L >= 1; --L) {
-    int cnt = 0;
-    for (int d = lane; d < n_docs; d += 32) cnt += (((cu[d + 1] - cu[d] + 127) >> 7) >= L) ? 1 : 0;
+    int cnt = nb0 >= L ? 1 : 0;
+    for (int d = lane + 32; d < n_docs; d += 32) cnt += (((cu[d + 1] - cu[d] + 127) >> 7) >= L) ? 1 : 0;
     const int tot = __reduce_add_sync(0xffffffffu, cnt);
     if (b < tot) {
       for (int d0 = 0; d0 < n_docs; d0 += 32) {        // the b-th document, in document order, with >= L blocks
         const int d = d0 + lane;
-        const bool has = d < n_docs && (((cu[d + 1] - cu[d] + 127) >> 7) >= L);
+        const bool has = d0 == 0 ? nb0 >= L : d < n_docs && (((cu[d + 1] - cu[d] + 127) >> 7) >= L);
         const unsigned m = __ballot_sync(0xffffffffu, has);
         const int c = __popc(m);
         if (b < c) {

@@ -13,10 +13,11 @@
 // S, O accumulated in TMEM, P consumed from TMEM, dedicated MMA and TMA warps, one
 // thread per score row, no CTA barrier in the loop); attn_fwd_kernel (first form:
 // 128-row kv blocks, O in registers) and attn_fwd2_kernel (two threads per row)
-// are kept for comparison (CB_ATTN_FWD=1 / 2).  Backward: attn_bwd2_kernel (one
-// CTA per kv block and head, two threads per score row, S / dP / dQ sharing TMEM
-// columns, dQ out by TMA reduce-add) with attn_delta_kernel before and
-// attn_bwd_finalize_kernel after it.
+// are kept for comparison (CB_ATTN_FWD=1 / 2).  Backward: one CTA per kv block and
+// head, dQ / dK / dV out by reduce-adds; attn_bwd3_kernel (one CTA an SM, every
+// product in flight beside the softmax, warps by role) or, for short documents of
+// head size 64, attn_bwd2_kernel (two CTAs an SM, one phase after another); with
+// attn_delta_kernel before and attn_bwd_finalize_kernel after it.
 //
 // Every thread that owns a score row reads it from TMEM with tcgen05.ld, so the
 // softmax needs no cross-thread shuffles.  The same swizzled image of a [128 x 64]
@@ -27,6 +28,7 @@
 // Replaces the reference's calls into flash-attn / SDPA (chronicals/kernels/
 // flash_attention_optimizer.py:845-994) and its forward-only Triton kernels
 // (:2460-3209); the reference has no attention backward of its own.
+#include <algorithm>
 #include <cstdlib>
 #include "common.cuh"
 
@@ -1044,8 +1046,8 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
 
 // ---------------------------------------------------------------------------------------------------
 // Backward.  One CTA: kv block `jb` of one document, one query head; loops over the query blocks i >= jb.
-// For D = 64 it needs 256 TMEM columns and ~97 KB of shared memory, so two CTAs share an SM and one computes
-// its softmax while the other has the tensor core (D = 128: 512 columns, 160 KB, one CTA per SM).
+// For D = 64 only (the rule between this and the pipelined form below stands at cb_attn_bwd): it needs 256 TMEM columns
+// and ~97 KB of shared memory, so two CTAs share an SM and one computes its softmax while the other has the tensor core.
 // The S, dP and dQ tiles take turns in the same 128 TMEM columns, and P and dS take turns in one shared
 // tile, which turns an iteration into three MMA phases:
 //   S = Q K^T            -> P = exp(S - lse)            (P to smem)
@@ -1056,13 +1058,11 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
 template <int D>
 struct Bwd2Smem {
   static constexpr int TILE = 128 * D * 2;
-  static constexpr int NQ = (D == 128) ? 2 : 1;       // Q / dO stages: D = 128 runs one CTA per SM and has the room to
-                                                      // fetch the next query block while this one is worked on
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = TILE;
-  static constexpr int OFF_Q = 2 * TILE;              // NQ stages
-  static constexpr int OFF_DO = (2 + NQ) * TILE;      // NQ stages
-  static constexpr int OFF_P = (2 + 2 * NQ) * TILE;   // P, then dS (bf16 [128 x 128] operand image)
+  static constexpr int OFF_Q = 2 * TILE;
+  static constexpr int OFF_DO = 3 * TILE;
+  static constexpr int OFF_P = 4 * TILE;              // P, then dS (bf16 [128 x 128] operand image)
   static constexpr int OFF_BAR = OFF_P + 32768;
   static constexpr int TOTAL = OFF_BAR + 128 + 1024;
 };
@@ -1088,7 +1088,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmdQ, const AttnArgs a) {
   using L = Bwd2Smem<D>;
   constexpr int PANELS = D / 64;
-  constexpr uint32_t TMEM_COLS = (128 + 2 * D) <= 256 ? 256 : 512;
+  constexpr uint32_t TMEM_COLS = 256;
+  static_assert(128 + 2 * D <= 256, "tensor memory of one CTA of two");
   constexpr uint32_t C_S = 0, C_DV = 128, C_DK = 128 + D;                // S, dP and dQ share the first 128 columns
   constexpr uint32_t IDESC_S = umma_idesc_bf16(128, 128, 0, 0);
   constexpr uint32_t IDESC_T = umma_idesc_bf16(128, D, 1, 1);            // P^T dO, dS^T Q
@@ -1107,14 +1108,13 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint8_t* sQ = smem + L::OFF_Q;
   uint8_t* sdO = smem + L::OFF_DO;
   uint8_t* sP = smem + L::OFF_P;
-  constexpr int NQ = L::NQ;
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);   // [2]
-  uint64_t* bar_kv = q_full + 2;
-  uint64_t* bar_s = q_full + 3;
-  uint64_t* bar_dp = q_full + 4;
-  uint64_t* bar_dq = q_full + 5;
-  uint64_t* stg_free = q_full + 6;                   // the dQ tile of the last iteration has left shared memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_full + 7);
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  uint64_t* bar_kv = q_full + 1;
+  uint64_t* bar_s = q_full + 2;
+  uint64_t* bar_dp = q_full + 3;
+  uint64_t* bar_dq = q_full + 4;
+  uint64_t* stg_free = q_full + 5;                   // the dQ tile of the last iteration has left shared memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_full + 6);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   // 8 warps: warps w and w + 4 own the same 32 TMEM lanes (score rows) and split the columns in halves,
@@ -1122,7 +1122,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int tid = threadIdx.x, warp = tid >> 5;
   const int q4 = warp & 3, half = warp >> 2;
   if (tid == 0) {
-    mbar_init(q_full, 1); mbar_init(q_full + 1, 1); mbar_init(bar_kv, 1); mbar_init(bar_s, 1); mbar_init(bar_dp, 1); mbar_init(bar_dq, 1);
+    mbar_init(q_full, 1); mbar_init(bar_kv, 1); mbar_init(bar_s, 1); mbar_init(bar_dp, 1); mbar_init(bar_dq, 1);
     mbar_init(stg_free, 1);
     mbar_fence_init();
     *abort_flag = a.status[0] != 0 ? 1 : 0;
@@ -1144,14 +1144,13 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int u_start = __shfl_sync(0xffffffffu, start, 0);
   const int u_jb = __shfl_sync(0xffffffffu, jb, 0);
   const int kv_row0 = u_start + u_jb * 128;
-  auto load_q = [&](int it) {                          // Q / dO of query block jb + it into stage it % NQ
+  auto load_q = [&](int it) {                          // Q / dO of query block jb + it
     const int row0 = u_start + (u_jb + it) * 128;
-    const int st = it % NQ;
-    mbar_expect_tx(q_full + st, 2 * L::TILE);
+    mbar_expect_tx(q_full, 2 * L::TILE);
 #pragma unroll
     for (int p = 0; p < PANELS; ++p) {
-      tma_load_2d(sQ + st * L::TILE + p * 16384, &tmQ, q_full + st, h * D + p * 64, row0);
-      tma_load_2d(sdO + st * L::TILE + p * 16384, &tmdO, q_full + st, h * D + p * 64, row0);
+      tma_load_2d(sQ + p * 16384, &tmQ, q_full, h * D + p * 64, row0);
+      tma_load_2d(sdO + p * 16384, &tmdO, q_full, h * D + p * 64, row0);
     }
   };
 
@@ -1171,7 +1170,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   const int r = q4 * 32 + (tid & 31);
   const float sl2 = a.scale * LOG2E;
-  const uint32_t kA = smem_u32(sK), vA = smem_u32(sV), pA = smem_u32(sP);
+  const uint32_t kA = smem_u32(sK), vA = smem_u32(sV), pA = smem_u32(sP), qA = smem_u32(sQ), doA = smem_u32(sdO);
   const uint32_t u_tmem = __shfl_sync(0xffffffffu, tmem, 0);
   // lse and delta of my query row: fetched one iteration ahead, the loads fly while this iteration works
   // (the loaded values are not touched before the next iteration, so nothing waits for the loads here)
@@ -1192,9 +1191,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   for (int it = 0; it < n_it; ++it) {
     const int i = jb + it;
     CB_PHASE(0);
-    const uint32_t qA = smem_u32(sQ + (it % NQ) * L::TILE), doA = smem_u32(sdO + (it % NQ) * L::TILE);
     if (w0) {
-      ok = __all_sync(0xffffffffu, mbar_wait(q_full + (it % NQ), (it / NQ) & 1, abort_flag, a.status, CB_ERR_WAIT_FULL) && ok);
+      ok = __all_sync(0xffffffffu, mbar_wait(q_full, it & 1, abort_flag, a.status, CB_ERR_WAIT_FULL) && ok);
       tc_fence_after();
       if (elect_one()) {
         if (ok) {
@@ -1203,10 +1201,9 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             umma_f16_ss(u_tmem + C_S, desc_kmajor(qA, kk), desc_kmajor(kA, kk), IDESC_S, kk != 0);
           umma_commit(bar_s);
         }
-        // While S is computed, the TMA reduce of the last iteration's dQ tile finishes reading the P / dS buffer
-        // (and, D = 128, the dO stage the next load goes to); everybody waits for `stg_free` before writing P.
+        // While S is computed, the TMA reduce of the last iteration's dQ tile finishes reading the P / dS buffer;
+        // everybody waits for `stg_free` before writing P.
         tma_store_wait_read<0>();
-        if (NQ == 2 && ok && it + 1 < n_it) load_q(it + 1);
         mbar_arrive(stg_free);
       }
     }
@@ -1266,7 +1263,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         umma_commit(bar_dp);
       }
     }
-    // ---- phase 2: dS = P (dP - delta) scale, overwriting P in shared memory
+    // ---- phase 2: dS = P (dP - delta), overwriting P in shared memory (the score scale is applied to dQ and dK at the end)
     CB_PHASE(5);
     ok &= mbar_wait(bar_dp, it & 1, abort_flag, a.status, CB_ERR_WAIT_TMEM_FULL);
     tc_fence_after();
@@ -1281,8 +1278,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
         const float2 pp = unpack_bf16x2(pk[cl][k]);
-        ds[k] = pack_bf16x2(pp.x * (__uint_as_float(dp[2 * k]) - dlt) * a.scale,
-                            pp.y * (__uint_as_float(dp[2 * k + 1]) - dlt) * a.scale);
+        ds[k] = pack_bf16x2(pp.x * (__uint_as_float(dp[2 * k]) - dlt),
+                            pp.y * (__uint_as_float(dp[2 * k + 1]) - dlt));
       }
       store_row_chunk32_packed(sP, r, c, ds);
     }
@@ -1308,22 +1305,20 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     ok &= mbar_wait(bar_dq, it & 1, abort_flag, a.status, CB_ERR_WAIT_TMEM_FULL);
     tc_fence_after();
     CB_PHASE(10);
-    if (NQ == 1 && w0 && ok && it + 1 < n_it) {                         // Q / dO of this iteration are consumed
+    if (w0 && ok && it + 1 < n_it) {                         // Q / dO of this iteration are consumed
       if (elect_one()) load_q(it + 1);
     }
     {
       // dQ tile (fp32) -> shared memory as [128 x 32] boxes in the layout of the dq_acc tensor map -> one TMA
-      // reduce-add per box instead of eight red.global.add per thread and box.  The first two boxes go to the
-      // P / dS buffer, which nobody reads any more; D = 128 has two more, which go to this iteration's dO stage
-      // (dV and dP have consumed it; the next load into that stage waits for the reduce's reads, see the loop top).
+      // reduce-add per box instead of eight red.global.add per thread and box.  The boxes go to the P / dS buffer,
+      // which nobody reads any more.
       // Rows past the end of the document carry exact zeros (their P was masked), rows past T are clipped.
-      uint8_t* sdO_it = sdO + (it % NQ) * L::TILE;
 #pragma unroll
       for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
         uint32_t dq[32];
         tmem_ld_32x32(t_row + C_S + c * 32, dq);
         tmem_ld_wait();
-        uint8_t* dstrow = (c < 2 ? sP + c * 16384 : sdO_it + (c - 2) * 16384) + r * 128;
+        uint8_t* dstrow = sP + c * 16384 + r * 128;
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc)
           *reinterpret_cast<uint4*>(dstrow + ((cc ^ (r & 7)) << 4)) = make_uint4(dq[4 * cc], dq[4 * cc + 1], dq[4 * cc + 2], dq[4 * cc + 3]);
@@ -1337,7 +1332,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         CB_DEBUG_CHECK_ST(a.status, start + i * 128 >= 0 && ((h * D) * 4) % 16 == 0, CB_DBG_TMA_COORD, start + i * 128);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c)
-          tma_reduce_add_2d(&tmdQ, c < 2 ? sP + c * 16384 : sdO_it + (c - 2) * 16384, h * D + c * 32,
+          tma_reduce_add_2d(&tmdQ, sP + c * 16384, h * D + c * 32,
                             u_start + (u_jb + it) * 128);
         tma_store_commit();
       }
@@ -1381,40 +1376,470 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
 }
 
-// dqkv[t] = bf16( dQ | sum over the query heads of a group of dK | same for dV ); one block per token,
-// four consecutive columns per thread (D is a multiple of 4, so a group never straddles heads)
-__global__ void attn_bwd_finalize_kernel(float* __restrict__ dq_acc, float* __restrict__ dk_part,
-                                         float* __restrict__ dv_part, bf16* __restrict__ dqkv, long long ld,
-                                         int T, int hq, int hk, int D, const int* __restrict__ cu, int n_docs,
-                                         int part_heads, int clear) {
-  // part_heads: heads per token in dk_part / dv_part — hq (one partial per query head, summed here) or hk
-  // (already accumulated per kv head by the kernel).  clear: write zeros back over every accumulator value read, so
-  // that a caller who keeps the scratch buffers between calls never has to clear them again.
-  const long long t = blockIdx.x;
-  const int nq = hq * D, nk = hk * D, g = part_heads / hk;
-  bf16* out = dqkv + t * ld;
-  const bool valid = t < cu[n_docs];                  // padding tokens get zero gradients
-  for (int c = threadIdx.x * 4; c < nq + 2 * nk; c += blockDim.x * 4) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid) {
-      if (c < nq) {
-        v = *reinterpret_cast<const float4*>(dq_acc + t * nq + c);
-        if (clear) *reinterpret_cast<float4*>(dq_acc + t * nq + c) = make_float4(0.f, 0.f, 0.f, 0.f);
-      } else {
-        const int cc = (c - nq) % nk, which = (c - nq) / nk;
-        const int kvh = cc / D, d = cc % D;
-        float* src = (which == 0 ? dk_part : dv_part) + (t * part_heads + static_cast<long long>(kvh) * g) * D + d;
-        for (int i = 0; i < g; ++i) {
-          const float4 x = *reinterpret_cast<const float4*>(src + static_cast<long long>(i) * D);
-          v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-          if (clear) *reinterpret_cast<float4*>(src + static_cast<long long>(i) * D) = make_float4(0.f, 0.f, 0.f, 0.f);
+// ---------------------------------------------------------------------------------------------------
+// Backward, pipelined form (D = 128, and D = 64 with few or long blocks).  One CTA: kv block `jb` of one document, one query head; loops over the query
+// blocks i >= jb.  The scores are kept transposed (rows = keys, S^T = K Q^T), so that P^T is an A operand straight from
+// TMEM and dS^T, written to shared memory once, serves as the K-major A operand of dK and as the MN-major one of dQ:
+//   S^T = K Q^T -> P^T -> dV += P^T dO;   dP^T = V dO^T -> dS^T -> dQ = dS K, dK += dS^T Q
+// At D = 128 the five products of an iteration read 288 KB of operands from shared memory and the rest moves 224 KB:
+// 4096 cycles at 128 bytes a cycle, against 2560 of the tensor core.  One phase after another (the form above, which D =
+// 128 used before) took 10,500; here the roles work on different products at the same time, each in its own warps:
+//   warps 0-7   P and dS: warps w and w + 4 share 32 keys and take 64 query columns each
+//   warps 8-11  dQ out of TMEM, 32 query rows each: all of it to registers at once, so that dP may follow, then through
+//               two 4 KB boxes a warp and TMA reduce-add
+//   warp 12     every MMA, in the order dV(i), S(i+1), dQ(i), dK(i), dP(i+1): while the tensor core has dV and S the
+//               softmax warps compute dS(i), while it has dQ, dK and dP they compute P(i+1)
+//   warp 13     TMA loads (Q two blocks deep, dO one) and the statistics of the query rows
+// TMEM: S^T [0, 128) with P^T over the first half of each 32 columns, dP^T [128, 256), dV, dK, and dQ over dP^T (D = 128)
+// or in columns of its own (D = 64, where dP need not wait for dQ to leave).
+// What bounds it now: 6600 cycles an iteration, of which the products with the waits between the roles take 5900 and the
+// softmax with them 5200 when the other is left out; the reduce-adds of dQ cost 60 us of 720.
+// Measured (kernel alone): 2 x 4096 tokens, 28 / 4 heads of 128: 1144 -> 721 us (526 -> 834 TFLOP/s); 27 documents in 8192
+// tokens, the same heads: 393 -> 274; 8 x 1024: 412 -> 310; 14 / 2 heads of 64: 1 x 2048 80 -> 44, 1 x 4096 160 -> 141.
+template <int D>
+struct Bwd3Smem {
+  static constexpr int TILE = 128 * D * 2;
+  static constexpr int OFF_K = 0;
+  static constexpr int OFF_V = TILE;
+  static constexpr int OFF_Q = 2 * TILE;              // 2 stages
+  static constexpr int NDO = D == 64 ? 2 : 1;         // dO stages
+  static constexpr int OFF_DO = 4 * TILE;
+  static constexpr int OFF_DS = (4 + NDO) * TILE;     // bf16 [128 keys x 128 queries] operand image
+  static constexpr int OFF_DQ = OFF_DS + 32768;       // 4 warps x 2 boxes of 32 rows x 32 fp32 columns
+  static constexpr int OFF_ST = OFF_DQ + 32768;       // 2 stages x (lse, delta) x 128 query rows
+  static constexpr int OFF_BAR = OFF_ST + 2048;
+  static constexpr int SLACK = 768;                   // for the alignment to 1024; the base is checked
+  static constexpr int TOTAL = OFF_BAR + 256 + SLACK;
+};
+static_assert(Bwd3Smem<128>::TOTAL <= 232448, "shared memory per CTA");
+static_assert(Bwd3Smem<128>::OFF_DQ - Bwd3Smem<128>::OFF_Q >= 8 * 4 * 4096 && Bwd3Smem<64>::OFF_DQ - Bwd3Smem<64>::OFF_Q >= 8 * 2 * 4096,
+              "boxes of dV and dK at the end");
+constexpr int BWD3_SOFTMAX_WARPS = 8;
+constexpr int BWD3_THREADS = 512;                     // warps 14 and 15 only complete the last warpgroup
+// registers a thread after the split: 256 x 144 + 128 x 144 + 128 x 80 = the 512 x 128 at launch
+constexpr int BWD3_REGS_SOFTMAX = 144, BWD3_REGS_DQ = 144, BWD3_REGS_ISSUE = 80;
+template <int N>
+__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+template <int D>
+__global__ void __launch_bounds__(BWD3_THREADS, 1)
+attn_bwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
+                 const __grid_constant__ CUtensorMap tmdQ, const __grid_constant__ CUtensorMap tmdK,
+                 const __grid_constant__ CUtensorMap tmdV, const AttnArgs a) {
+  using L = Bwd3Smem<D>;
+  constexpr int PANELS = D / 64;
+  constexpr uint32_t TMEM_COLS = 512;
+  constexpr bool DQ_APART = D == 64;                   // columns are left for a dQ of its own
+  constexpr uint32_t C_S = 0, C_DP = 128, C_DQ = DQ_APART ? 256 + 2 * D : 128, C_DV = 256, C_DK = 256 + D;
+  constexpr int NDO = L::NDO;
+  constexpr uint32_t IDESC_S = umma_idesc_bf16(128, 128, 0, 0);          // K Q^T, V dO^T
+  constexpr uint32_t IDESC_KV = umma_idesc_bf16(128, D, 0, 1);           // P^T dO, dS^T Q
+  constexpr uint32_t IDESC_DQ = umma_idesc_bf16(128, D, 1, 1);           // dS K
+
+  int start, len, jb, nblk;
+  if (!locate_tile(a.cu, a.n_docs, blockIdx.y, start, len, jb, nblk)) return;
+  jb = nblk - jb;                                      // weight = query blocks from the diagonal on = nblk - jb
+  const int h = blockIdx.x;
+  const int hkv = h / (a.hq / a.hk);
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sK = smem + L::OFF_K;
+  uint8_t* sV = smem + L::OFF_V;
+  uint8_t* sQ = smem + L::OFF_Q;
+  uint8_t* sdO = smem + L::OFF_DO;
+  uint8_t* sdS = smem + L::OFF_DS;
+  float* sStat = reinterpret_cast<float*>(smem + L::OFF_ST);             // [stage][lse * log2(e) | delta][128]
+  uint64_t* k_full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  uint64_t* v_full = k_full + 1;
+  uint64_t* q_full = v_full + 1;                      // [2]
+  uint64_t* q_empty = q_full + 2;                      // [2] dK(i) complete
+  uint64_t* st_full = q_empty + 2;                     // [2] statistics written (free with the Q stage)
+  uint64_t* do_full = st_full + 2;                     // [2]
+  uint64_t* do_empty = do_full + 2;                    // [2] dV(i) complete
+  uint64_t* s_full = do_empty + 2;                     // S(i) complete
+  uint64_t* p_ready = s_full + 1;                      // an arrival per softmax warp: S(i) read, P(i) in TMEM
+  uint64_t* dp_full = p_ready + 1;                     // dP(i) complete
+  uint64_t* ds_ready = dp_full + 1;                    // the same: dP(i) read, dS(i) in shared memory
+  uint64_t* ds_free = ds_ready + 1;                    // dQ(i) and dK(i) complete
+  uint64_t* dq_full = ds_free + 1;                     // dQ(i) complete
+  uint64_t* dq_free = dq_full + 1;                     // 4 arrivals: dQ(i) out of TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_free + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  if (smem - smem_raw > L::SLACK) {                    // the same in every thread and every CTA
+    if (tid == 0) atomicCAS(a.status, 0, CB_ERR_WAIT_MISC);
+    return;
+  }
+  if (tid == 0) {
+    mbar_init(k_full, 1); mbar_init(v_full, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(q_full + i, 1); mbar_init(q_empty + i, 1); mbar_init(st_full + i, 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(do_full + i, 1); mbar_init(do_empty + i, 1); }
+    mbar_init(s_full, 1); mbar_init(p_ready, BWD3_SOFTMAX_WARPS);
+    mbar_init(dp_full, 1); mbar_init(ds_ready, BWD3_SOFTMAX_WARPS); mbar_init(ds_free, 1); mbar_init(dq_full, 1); mbar_init(dq_free, 4);
+    mbar_fence_init();
+    *abort_flag = a.status[0] != 0 ? 1 : 0;
+  }
+  __syncthreads();
+  if (*abort_flag) return;
+  if (warp == 0) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int n_it = nblk - jb;
+  const int lane = tid & 31;
+  bool ok = true;
+  // one arrival for a warp: what its lanes did before is ordered by the warp barrier
+  auto arrive_w = [&](uint64_t* bar) {
+    __syncwarp();
+    if (elect_one()) mbar_arrive(bar);
+  };
+  CB_PHASE_DECL_T(384, 0);             // slot 0: the MMA warp, slot 1: a softmax thread
+  // every wait ends in a warp-wide vote, so that the lanes of a warp leave their loop together
+  auto wait_w = [&](uint64_t* bar, int phase, int code) {
+    ok = __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, abort_flag, a.status, code) && ok);
+    return ok;
+  };
+
+  if (warp >= 14) {
+    reg_dec<BWD3_REGS_ISSUE>();
+  } else if (warp == 13) {
+    reg_dec<BWD3_REGS_ISSUE>();
+    // ------------------------------------------------------------------ loads
+    const int u_start = __shfl_sync(0xffffffffu, start, 0);
+    const int u_jb = __shfl_sync(0xffffffffu, jb, 0);
+    const int u_n = __shfl_sync(0xffffffffu, n_it, 0);
+    float lse_n[4], dlt_n[4];                          // statistics of the next block: the loads fly an iteration ahead
+    auto fetch_stats = [&](int it) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int rg = (u_jb + it) * 128 + lane + 32 * k;
+        const long long at = static_cast<long long>(h) * a.T + u_start + rg;
+        const bool in = it < u_n && rg < len;
+        lse_n[k] = in ? __ldg(a.lse + at) : 0.f;
+        dlt_n[k] = in ? __ldg(a.delta + at) : 0.f;
+      }
+    };
+    fetch_stats(0);
+    if (elect_one()) {
+      mbar_expect_tx(k_full, L::TILE);                 // K and Q first: S(0) needs no more
+#pragma unroll
+      for (int p = 0; p < PANELS; ++p) tma_load_2d(sK + p * 16384, &tmK, k_full, hkv * D + p * 64, u_start + u_jb * 128);
+    }
+    for (int it = 0; it < u_n; ++it) {
+      const int st = it & 1;
+      const int row0 = u_start + (u_jb + it) * 128;
+      if (it >= 2 && !wait_w(q_empty + st, (it >> 1) - 1, CB_ERR_WAIT_EMPTY)) break;
+      if (elect_one()) {
+        mbar_expect_tx(q_full + st, L::TILE);
+#pragma unroll
+        for (int p = 0; p < PANELS; ++p) tma_load_2d(sQ + st * L::TILE + p * 16384, &tmQ, q_full + st, h * D + p * 64, row0);
+        if (it == 0) {
+          mbar_expect_tx(v_full, L::TILE);
+#pragma unroll
+          for (int p = 0; p < PANELS; ++p) tma_load_2d(sV + p * 16384, &tmV, v_full, hkv * D + p * 64, row0);
+        }
+      }
+      // rows past the end of the document get lse = +inf: their probabilities are exact zeros
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool in = (u_jb + it) * 128 + lane + 32 * k < len;
+        sStat[st * 256 + lane + 32 * k] = in ? lse_n[k] * LOG2E : INFINITY;
+        sStat[st * 256 + 128 + lane + 32 * k] = dlt_n[k];
+      }
+      arrive_w(st_full + st);
+      fetch_stats(it + 1);
+      const int sd = it % NDO;
+      if (it >= NDO && !wait_w(do_empty + sd, it / NDO - 1, CB_ERR_WAIT_EMPTY)) break;
+      if (elect_one()) {
+        mbar_expect_tx(do_full + sd, L::TILE);
+#pragma unroll
+        for (int p = 0; p < PANELS; ++p) tma_load_2d(sdO + sd * L::TILE + p * 16384, &tmdO, do_full + sd, h * D + p * 64, row0);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 12) {
+    reg_dec<BWD3_REGS_ISSUE>();
+    // ------------------------------------------------------------------ MMA issue
+    const int u_n = __shfl_sync(0xffffffffu, n_it, 0);
+    const uint32_t u_tmem = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t kA = smem_u32(sK), vA = smem_u32(sV), dsA = smem_u32(sdS);
+    auto issue_s = [&](int it) {                       // S^T(it) = K Q(it)^T
+      if (!wait_w(q_full + (it & 1), it >> 1, CB_ERR_WAIT_FULL)) return;
+      const uint32_t qA = smem_u32(sQ + (it & 1) * L::TILE);
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk)
+          umma_f16_ss(u_tmem + C_S, desc_kmajor(kA, kk), desc_kmajor(qA, kk), IDESC_S, kk != 0);
+        umma_commit(s_full);
+      }
+    };
+    auto issue_dp = [&](int it) {                      // dP^T(it) = V dO(it)^T
+      if (!wait_w(do_full + it % NDO, it / NDO, CB_ERR_WAIT_FULL)) return;
+      const uint32_t doA = smem_u32(sdO + (it % NDO) * L::TILE);
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk)
+          umma_f16_ss(u_tmem + C_DP, desc_kmajor(vA, kk), desc_kmajor(doA, kk), IDESC_S, kk != 0);
+        umma_commit(dp_full);
+      }
+    };
+    wait_w(k_full, 0, CB_ERR_WAIT_FULL);
+    if (ok) issue_s(0);
+    if (ok && wait_w(v_full, 0, CB_ERR_WAIT_FULL)) issue_dp(0);
+    CB_PHASE(12);
+    for (int it = 0; it < u_n && ok; ++it) {
+      if (!wait_w(p_ready, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
+      CB_PHASE(0);
+      const uint32_t doA = smem_u32(sdO + (it % NDO) * L::TILE);
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                 // dV += P^T dO, A from TMEM: 16 queries = 8 words a step
+          umma_f16_ts(u_tmem + C_DV, u_tmem + C_S + (kk >> 1) * 32 + (kk & 1) * 8, desc_mnmajor(doA, kk), IDESC_KV, (it | kk) != 0);
+        umma_commit(do_empty + it % NDO);
+      }
+      if (it + 1 < u_n) issue_s(it + 1);               // over S(it), P(it): both are consumed, MMAs complete in order
+      CB_PHASE(1);
+      if (!ok || !wait_w(ds_ready, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
+      CB_PHASE(2);
+      if (DQ_APART) {                                  // dP(it + 1) needs nothing of this dQ: first, so that dS is not kept waiting
+        if (it + 1 < u_n) issue_dp(it + 1);
+        if (!ok || (it > 0 && !wait_w(dq_free, it - 1, CB_ERR_WAIT_TMEM_EMPTY))) break;
+      }
+      const uint32_t qA = smem_u32(sQ + (it & 1) * L::TILE);
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                 // dQ = dS K (D = 128: over the columns of dP)
+          umma_f16_ss(u_tmem + C_DQ, desc_mnmajor(dsA, kk), desc_mnmajor(kA, kk), IDESC_DQ, kk != 0);
+        umma_commit(dq_full);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                 // dK += dS^T Q
+          umma_f16_ss(u_tmem + C_DK, desc_kmajor(dsA, kk), desc_mnmajor(qA, kk), IDESC_KV, (it | kk) != 0);
+        umma_commit(ds_free);
+        umma_commit(q_empty + (it & 1));
+      }
+      CB_PHASE(3);
+      if (!DQ_APART && it + 1 < u_n) {
+        if (!wait_w(dq_free, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
+        CB_PHASE(4);
+        issue_dp(it + 1);
+        CB_PHASE(5);
+      }
+    }
+    __syncwarp();
+  } else if (warp >= 8) {
+    reg_inc<BWD3_REGS_DQ>();
+    // ------------------------------------------------------------------ dQ: TMEM -> shared memory -> TMA reduce-add
+    // Rows past the end of the document belong to the next one and get zeros; a box of nothing else stays here.
+    const int q4 = warp - BWD3_SOFTMAX_WARPS;
+    const uint32_t t_row = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
+    uint8_t* box = smem + L::OFF_DQ + q4 * 8192;
+    for (int it = 0; it < n_it; ++it) {
+      if (!wait_w(dq_full, it, CB_ERR_WAIT_TMEM_FULL)) break;
+      tc_fence_after();
+uint32_t dq[D / 32][32];
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) tmem_ld_32x32(t_row + C_DQ + c * 32, dq[c]);
+      tmem_ld_wait();
+      tc_fence_before();
+      arrive_w(dq_free);
+      if ((jb + it) * 128 + q4 * 32 + lane >= len) {   // rows of the next document: nothing, whatever either holds
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c)
+#pragma unroll
+          for (int k = 0; k < 32; ++k) dq[c][k] = 0u;
+      }
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        if (elect_one()) tma_store_wait_read<1>();     // the box's reduce before last has been read
+        __syncwarp();
+        uint8_t* row = box + (c & 1) * 4096 + lane * 128;
+#pragma unroll
+        for (int cc = 0; cc < 8; ++cc)
+          *reinterpret_cast<uint4*>(row + ((cc ^ (lane & 7)) << 4)) =
+              make_uint4(dq[c][4 * cc], dq[c][4 * cc + 1], dq[c][4 * cc + 2], dq[c][4 * cc + 3]);
+        fence_async_smem();
+        __syncwarp();
+        if (elect_one()) {
+          CB_DEBUG_CHECK_ST(a.status, start + (jb + it) * 128 >= 0, CB_DBG_TMA_COORD, start + (jb + it) * 128);
+          if ((jb + it) * 128 + q4 * 32 < len)
+            tma_reduce_add_2d(&tmdQ, box + (c & 1) * 4096, h * D + c * 32, start + (jb + it) * 128 + q4 * 32);
+          tma_store_commit();
         }
       }
     }
-    uint2 o;
-    o.x = pack_bf16x2(v.x, v.y);
-    o.y = pack_bf16x2(v.z, v.w);
-    *reinterpret_cast<uint2*>(out + c) = o;
+    if (elect_one()) tma_store_wait_read<0>();
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ P and dS: my key r, 64 query columns
+    reg_inc<BWD3_REGS_SOFTMAX>();
+    const int q4 = warp & 3, half = warp >> 2;
+    const int r = q4 * 32 + lane;
+    const uint32_t t_row = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
+    const uint32_t t_s = t_row + C_S + half * 64, t_dp = t_row + C_DP + half * 64;
+    const float sl2 = a.scale * LOG2E;
+    CB_PHASE(12);
+    for (int it = 0; it < n_it; ++it) {
+      const float4* lse4 = reinterpret_cast<const float4*>(sStat + (it & 1) * 256 + half * 64);
+      const float4* dlt4 = lse4 + 32;
+      if (!wait_w(st_full + (it & 1), it >> 1, CB_ERR_WAIT_FULL)) break;
+      CB_PHASE(0);
+      if (!wait_w(s_full, it, CB_ERR_WAIT_TMEM_FULL)) break;
+      CB_PHASE(1);
+      tc_fence_after();
+      uint32_t pk[2][16];
+      {
+        uint32_t s[2][32];
+        tmem_ld_32x32(t_s, s[0]);
+        tmem_ld_32x32(t_s + 32, s[1]);
+        tmem_ld_wait();
+        if (it == 0) {                                 // the diagonal block: queries before my key see nothing of it
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            if (half * 64 + c < r) s[0][c] = 0xff800000u;                // -inf
+            if (half * 64 + 32 + c < r) s[1][c] = 0xff800000u;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float4 l = lse4[c * 8 + k];
+            const float e0 = ex2_approx(fmaf(__uint_as_float(s[c][4 * k]), sl2, -l.x)), e1 = ex2_approx(fmaf(__uint_as_float(s[c][4 * k + 1]), sl2, -l.y));
+            const float e2 = ex2_approx(fmaf(__uint_as_float(s[c][4 * k + 2]), sl2, -l.z));
+            const float e3 = ex2_fma(fmaf(__uint_as_float(s[c][4 * k + 3]), sl2, -l.w));      // one in four on the FMA pipe
+            pk[c][2 * k] = pack_bf16x2(e0, e1);
+            pk[c][2 * k + 1] = pack_bf16x2(e2, e3);
+          }
+          tmem_st_32x16(t_s + c * 32, pk[c]);
+        }
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      arrive_w(p_ready);
+      CB_PHASE(2);
+      if (!wait_w(dp_full, it, CB_ERR_WAIT_TMEM_FULL)) break;
+      CB_PHASE(3);
+      tc_fence_after();
+      {                                                // dS = P (dP - delta), over pk
+        uint32_t dp[2][32];
+        tmem_ld_32x32(t_dp, dp[0]);
+        tmem_ld_32x32(t_dp + 32, dp[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float4 d = dlt4[c * 8 + k];
+            const float2 p0 = unpack_bf16x2(pk[c][2 * k]), p1 = unpack_bf16x2(pk[c][2 * k + 1]);
+            pk[c][2 * k] = pack_bf16x2(p0.x * (__uint_as_float(dp[c][4 * k]) - d.x), p0.y * (__uint_as_float(dp[c][4 * k + 1]) - d.y));
+            pk[c][2 * k + 1] = pack_bf16x2(p1.x * (__uint_as_float(dp[c][4 * k + 2]) - d.z), p1.y * (__uint_as_float(dp[c][4 * k + 3]) - d.w));
+          }
+        }
+      }
+      CB_PHASE(4);
+      if (it > 0 && !wait_w(ds_free, it - 1, CB_ERR_WAIT_MISC)) break;
+      CB_PHASE(5);
+      store_row_chunk32_packed(sdS, r, half * 2, pk[0]);
+      store_row_chunk32_packed(sdS, r, half * 2 + 1, pk[1]);
+      tc_fence_before();
+      fence_async_smem();
+      arrive_w(ds_ready);
+      CB_PHASE(6);
+    }
+    // dV and dK are added per kv head (the query heads of a group are different CTAs): [32 x 32] boxes in the Q, dO and dS
+    // tiles, which nothing reads any more, and a TMA reduce-add each.
+    if (ok && wait_w(ds_free, n_it - 1, CB_ERR_WAIT_MISC)) {
+      tc_fence_after();
+      constexpr int NB = D / 64;                       // chunks of 32 columns of either that are this warp's
+      uint8_t* box = sQ + warp * 2 * NB * 4096;        // 8 warps x 2 NB boxes from the Q tiles on
+#pragma unroll
+      for (int b = 0; b < 2 * NB; ++b) {
+        const int c = half * NB + b % NB;
+        uint32_t v[32];
+        tmem_ld_32x32(t_row + (b < NB ? C_DV : C_DK) + c * 32, v);
+        tmem_ld_wait();
+        if (jb * 128 + r >= len) {                     // keys of the next document: nothing, whatever either holds
+#pragma unroll
+          for (int k = 0; k < 32; ++k) v[k] = 0u;
+        }
+        uint8_t* row = box + b * 4096 + lane * 128;
+#pragma unroll
+        for (int cc = 0; cc < 8; ++cc)
+          *reinterpret_cast<uint4*>(row + ((cc ^ (lane & 7)) << 4)) = make_uint4(v[4 * cc], v[4 * cc + 1], v[4 * cc + 2], v[4 * cc + 3]);
+      }
+      fence_async_smem();
+      __syncwarp();
+      const int row0 = jb * 128 + q4 * 32;             // the warp's first key within the document
+      if (row0 < len && elect_one()) {
+#pragma unroll
+        for (int b = 0; b < 2 * NB; ++b)
+          tma_reduce_add_2d(b < NB ? &tmdV : &tmdK, box + b * 4096, hkv * D + (half * NB + b % NB) * 32, start + row0);
+        tma_store_commit();
+        tma_store_wait_read<0>();                      // shared memory is released when the CTA exits
+      }
+      __syncwarp();
+    }
+  }
+  CB_PHASE(11);
+  CB_PHASE_FLUSH;
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
+}
+
+// dqkv[t] = bf16( scale dQ | scale dK | dV ): the accumulators hold the gradients without the score scale, which is
+// cheaper to apply here, once a value, than to every dS.  Bound by memory (two reads of 4 bytes a value for one write
+// of 2): a thread takes 8 columns (D is a multiple of 8, so they lie in one section), ATT_FIN_BATCH of them at a time.
+// 8192 tokens, 28 / 4 heads of 128: 32 us (7 TB/s) against 50 with one float4 in flight.
+// clear: write zeros back over every accumulator value read, so that a caller who keeps the scratch buffers between
+// calls never has to clear them again.
+constexpr int ATT_FIN_BATCH = 3;
+__global__ void __launch_bounds__(256)
+attn_bwd_finalize_kernel(float* __restrict__ dq_acc, float* __restrict__ dk_part, float* __restrict__ dv_part,
+                         bf16* __restrict__ dqkv, long long ld, int nq, int nk, float scale, const int* __restrict__ cu,
+                         int n_docs, int clear) {
+  const long long t = blockIdx.x;
+  const int total = (nq + 2 * nk) / 8;
+  uint4* out = reinterpret_cast<uint4*>(dqkv + t * ld);
+  const bool valid = t < cu[n_docs];                  // padding tokens get zero gradients
+  for (int c0 = threadIdx.x; c0 < total; c0 += ATT_FIN_BATCH * blockDim.x) {
+    float4 v[ATT_FIN_BATCH][2];
+#pragma unroll
+    for (int i = 0; i < ATT_FIN_BATCH; ++i) {
+      const int c = (c0 + i * blockDim.x) * 8;
+      v[i][0] = v[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (valid && c < nq + 2 * nk) {
+        float4* src = reinterpret_cast<float4*>(c < nq ? dq_acc + t * nq + c
+                                                       : c < nq + nk ? dk_part + t * nk + (c - nq) : dv_part + t * nk + (c - nq - nk));
+        v[i][0] = src[0];
+        v[i][1] = src[1];
+        if (clear) src[0] = src[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < ATT_FIN_BATCH; ++i) {
+      const int c = (c0 + i * blockDim.x) * 8;
+      if (c < nq + 2 * nk) {
+        const float m = c < nq + nk ? scale : 1.f;
+        out[c / 8] = make_uint4(pack_bf16x2(v[i][0].x * m, v[i][0].y * m), pack_bf16x2(v[i][0].z * m, v[i][0].w * m),
+                                pack_bf16x2(v[i][1].x * m, v[i][1].y * m), pack_bf16x2(v[i][1].z * m, v[i][1].w * m));
+      }
+    }
   }
 }
 
@@ -1514,6 +1939,7 @@ int cb_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
                 long long ldo, long long ld_do, float scale, float* delta, float* dq_acc, float* dk_part,
                 float* dv_part, void* dqkv, long long ld_dqkv, int* status, void* stream, int scratch_is_zero) {
   if ((D != 64 && D != 128) || hq % hk != 0 || T <= 0 || n_docs <= 0) return -1;
+  if ((reinterpret_cast<uintptr_t>(dqkv) & 15) != 0 || ld_dqkv % 8 != 0) return -1;
   CUtensorMap mq, mk, mv, mdo;
   int e = attn_maps(&mq, &mk, &mv, q, k, v, T, hq, hk, D, ldq, ldk, ldv);
   if (e) return e;
@@ -1554,20 +1980,38 @@ int cb_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
   a.lse = const_cast<float*>(lse); a.delta = delta; a.dq_acc = dq_acc; a.dk_part = dk_part; a.dv_part = dv_part;
   a.status = status;
   dim3 grid(hq, (T + 127) / 128 + n_docs);            // x: query head (fastest, the heads of a group share K/V in L2); y: tile by descending weight
-  // Two threads per score row, S / dP / dQ sharing TMEM columns, dK / dV accumulated per kv head with red.add
-  // (so those buffers start from zero).  D = 64 additionally fits two CTAs per SM.
-  const int part_heads = hk;
-  if (D == 64) {
+  // D = 64 runs two CTAs of the phase-by-phase kernel on an SM where one of the pipelined kernel fits, so the pipelined one
+  // wins where the grid does not fill the SMs twice over (1 x 2048 tokens, 14 heads: 44 against 80 us; 4 x 512: 23 / 26)
+  // or its loops are long (2 x 4096: 276 / 290; 4 x 2048, 32 heads: 403 / 350, so no earlier than 4096), unless the
+  // documents are so short that a CTA is mostly set-up (20 x 100: 19 / 15).  Lengths as the average over the documents.
+  const bool few = static_cast<long long>(hq) * ((T + 127) / 128) <= 2LL * cbhost::num_sms() && T >= 512LL * n_docs;
+  if (D == 64 && !few && T < 4096LL * n_docs) {
     static bool cfg = false;
     if (!cfg) { e = set_smem(cb::attn_bwd2_kernel<64>, cb::Bwd2Smem<64>::TOTAL); if (e) return e; cfg = true; }
     cb::attn_bwd2_kernel<64><<<grid, cb::BWD2_THREADS, cb::Bwd2Smem<64>::TOTAL, s>>>(mq, mk, mv, mdo, mdq, a);
   } else {
-    static bool cfg = false;
-    if (!cfg) { e = set_smem(cb::attn_bwd2_kernel<128>, cb::Bwd2Smem<128>::TOTAL); if (e) return e; cfg = true; }
-    cb::attn_bwd2_kernel<128><<<grid, cb::BWD2_THREADS, cb::Bwd2Smem<128>::TOTAL, s>>>(mq, mk, mv, mdo, mdq, a);
+    CUtensorMap mdq32;                                  // the accumulator in boxes of 32 rows, one warp's share
+    e = cbhost::make_tmap(&mdq32, dq_acc, static_cast<unsigned long long>(hq) * D, T, static_cast<unsigned long long>(hq) * D,
+                          32, 32, 4);
+    if (e) return e;
+    CUtensorMap mdk, mdv;
+    e = cbhost::make_tmap(&mdk, dk_part, static_cast<unsigned long long>(hk) * D, T, static_cast<unsigned long long>(hk) * D, 32, 32, 4);
+    if (e) return e;
+    e = cbhost::make_tmap(&mdv, dv_part, static_cast<unsigned long long>(hk) * D, T, static_cast<unsigned long long>(hk) * D, 32, 32, 4);
+    if (e) return e;
+    if (D == 64) {
+      static bool cfg = false;
+      if (!cfg) { e = set_smem(cb::attn_bwd3_kernel<64>, cb::Bwd3Smem<64>::TOTAL); if (e) return e; cfg = true; }
+      cb::attn_bwd3_kernel<64><<<grid, cb::BWD3_THREADS, cb::Bwd3Smem<64>::TOTAL, s>>>(mq, mk, mv, mdo, mdq32, mdk, mdv, a);
+    } else {
+      static bool cfg = false;
+      if (!cfg) { e = set_smem(cb::attn_bwd3_kernel<128>, cb::Bwd3Smem<128>::TOTAL); if (e) return e; cfg = true; }
+      cb::attn_bwd3_kernel<128><<<grid, cb::BWD3_THREADS, cb::Bwd3Smem<128>::TOTAL, s>>>(mq, mk, mv, mdo, mdq32, mdk, mdv, a);
+    }
   }
-  cb::attn_bwd_finalize_kernel<<<T, 128, 0, s>>>(dq_acc, dk_part, dv_part, static_cast<cb::bf16*>(dqkv), ld_dqkv, T,
-                                                  hq, hk, D, cu, n_docs, part_heads, scratch_is_zero ? 1 : 0);
+  const int vecs = (hq + 2 * hk) * D / 8;
+  cb::attn_bwd_finalize_kernel<<<T, std::min(256, (vecs + cb::ATT_FIN_BATCH * 32 - 1) / (cb::ATT_FIN_BATCH * 32) * 32), 0, s>>>(
+      dq_acc, dk_part, dv_part, static_cast<cb::bf16*>(dqkv), ld_dqkv, hq * D, hk * D, scale, cu, n_docs, scratch_is_zero ? 1 : 0);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -100,47 +100,122 @@ __device__ __forceinline__ int mx_scale_exp(float amax, float fmt_max) {
   const int e = (mant == 0.5f) ? ex - 1 : ex;
   return max(-127, min(127, e));
 }
+// MXFP8 copies of x [R, C] and of its TRANSPOSE from one read of x: q_row [R, C] with blocks of 32 along C, q_col [C, R]
+// with blocks of 32 along R (what the products over one and over the other dimension contract over), both with packed
+// scales; either may be left out.  Bound by memory (2 bytes in, 2 out a value).  A block takes a tile of 128 x 128 to
+// shared memory with eight 16-byte loads a thread in flight, then quantises it twice: a thread takes 32 values of a row
+// (four neighbours: 128 contiguous bytes of q_row), and 32 rows of two neighbouring columns (four neighbours: 128
+// contiguous bytes of either row of q_col, where a thread per column wrote scattered 32-byte pieces).  The pitch of 264
+// bytes and the rotations below keep both kinds of access free of bank conflicts.
+// Measured, both copies of 4096 x 37,888 (e5m2): 124 us (5.0 TB/s), against 78 of a kernel for the rows and 109 of one for
+// the transpose that read x twice; of 37,888 x 3584 and 4096 x 3584 together (e4m3): 128 against 202.
+constexpr int MX_T = 128;                              // tile edge
+constexpr int MX_PITCH = MX_T * 2 + 8;
+
 // byte index of the scale of (row, block kb) in the packed atoms (rows grouped in tiles of tile_rows)
-__device__ __forceinline__ long long mx_sf_index(long long row, int kb, int kb4, int tile_rows) {
-  const long long tile = row / tile_rows;
-  const long long mp = tile * ((tile_rows + 127) / 128 * 128) + (row - tile * tile_rows);
-  return ((mp >> 7) * kb4 + (kb >> 2)) * 512 + (mp & 31) * 16 + ((mp >> 5) & 3) * 4 + (kb & 3);
+__device__ __forceinline__ size_t mx_sf_index(unsigned row, unsigned kb, unsigned kb4, unsigned tile_rows) {
+  const unsigned tile = row / tile_rows;
+  const unsigned mp = tile * ((tile_rows + 127) / 128 * 128) + (row - tile * tile_rows);
+  return (static_cast<size_t>(mp >> 7) * kb4 + (kb >> 2)) * 512 + (mp & 31) * 16 + ((mp >> 5) & 3) * 4 + (kb & 3);
+}
+template <int E5M2>
+__device__ __forceinline__ uint32_t mx_pack4(float a, float b, float c, float d) {
+  const __nv_fp8_interpretation_t f = E5M2 ? __NV_E5M2 : __NV_E4M3;
+  const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, f);
+  const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, f);
+  return static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
 }
 
-// MXFP8 copy of the TRANSPOSE of x [R, C] (bf16): q_col [C, R] with blocks of 32 along R (the dimension a
-// gradient GEMM contracts over) and packed scales for rows c, without materialising a bf16 transpose.
-// A block owns 32 rows x 256 columns; thread t owns column c0 + t, keeps its 32 values (one whole scale
-// block) in registers, and writes them as 32 contiguous bytes of row c of the output.
 template <int E5M2>
 __global__ void __launch_bounds__(256)
-mxfp8_quant_transposed_kernel(const bf16* __restrict__ x, long long R, int C, long long ldx,
-                              unsigned char* __restrict__ q_col, unsigned char* __restrict__ sf_col, int col_tile) {
+mxfp8_quant_dual_kernel(const bf16* __restrict__ x, int R, int C, long long ldx, unsigned char* __restrict__ q_row,
+                        unsigned char* __restrict__ sf_row, int row_tile, unsigned char* __restrict__ q_col,
+                        unsigned char* __restrict__ sf_col, int col_tile) {
+  __shared__ __align__(16) unsigned char tile[MX_T * MX_PITCH];
   const float fmt_max = E5M2 ? 57344.f : 448.f;
-  const long long r0 = static_cast<long long>(blockIdx.y) * 32;
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c >= C) return;
-  float v[32];
+  const int c0 = blockIdx.x * MX_T, r0 = blockIdx.y * MX_T;
+  const int tid = threadIdx.x;
+  {
+    const int cv = (tid & 15) * 8, r = tid >> 4;       // 16 lanes a row, 16 rows at a time
+    uint4 u[8];
 #pragma unroll
-  for (int r = 0; r < 32; ++r) v[r] = __bfloat162float(x[(r0 + r) * ldx + c]);
-  float amax = 0.f;
+    for (int i = 0; i < 8; ++i) {
+      const int rr = r + 16 * i;
+      u[i] = r0 + rr < R && c0 + cv < C ? *reinterpret_cast<const uint4*>(x + static_cast<long long>(r0 + rr) * ldx + c0 + cv)
+                                        : make_uint4(0u, 0u, 0u, 0u);
+    }
 #pragma unroll
-  for (int r = 0; r < 32; ++r) amax = fmaxf(amax, fabsf(v[r]));
-  const int e = mx_scale_exp(amax, fmt_max);
-  const float inv = exp2f(static_cast<float>(-e));
-  sf_col[mx_sf_index(c, static_cast<int>(r0 >> 5), static_cast<int>((R + 127) / 128), col_tile)] =
-      static_cast<unsigned char>(e + 127);
-  uint32_t w[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const __nv_fp8x2_storage_t p0 = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * i] * inv, v[4 * i + 1] * inv),
-                                                             __NV_SATFINITE, E5M2 ? __NV_E5M2 : __NV_E4M3);
-    const __nv_fp8x2_storage_t p1 = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * i + 2] * inv, v[4 * i + 3] * inv),
-                                                             __NV_SATFINITE, E5M2 ? __NV_E5M2 : __NV_E4M3);
-    w[i] = static_cast<uint32_t>(p0) | (static_cast<uint32_t>(p1) << 16);
+    for (int i = 0; i < 8; ++i) {
+      uint2* d = reinterpret_cast<uint2*>(tile + (r + 16 * i) * MX_PITCH + cv * 2);
+      d[0] = make_uint2(u[i].x, u[i].y);
+      d[1] = make_uint2(u[i].z, u[i].w);
+    }
   }
-  uint4* dst = reinterpret_cast<uint4*>(q_col + static_cast<long long>(c) * R + r0);
-  dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  __syncthreads();
+  if (q_row != nullptr) {
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+      const int kb = tid & 3, r = (tid >> 2) + 64 * pass;
+      // blocks 2 and 3 of a row start in their second half: 16 lanes then touch 32 different banks
+      const int turn = kb >> 1;
+      float v[32], amax = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint2 w = *reinterpret_cast<const uint2*>(tile + r * MX_PITCH + kb * 64 + ((j + 4 * turn) & 7) * 8);
+        const float2 a = unpack_bf16x2(w.x), b = unpack_bf16x2(w.y);
+        v[4 * j] = a.x; v[4 * j + 1] = a.y; v[4 * j + 2] = b.x; v[4 * j + 3] = b.y;
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))));
+      }
+      if (r0 + r < R && c0 + kb * 32 < C) {
+        const int e = mx_scale_exp(amax, fmt_max);
+        const float inv = exp2f(static_cast<float>(-e));
+        sf_row[mx_sf_index(r0 + r, c0 / 32 + kb, (C + 127) / 128, row_tile)] = static_cast<unsigned char>(e + 127);
+        uint32_t o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = mx_pack4<E5M2>(v[4 * j] * inv, v[4 * j + 1] * inv, v[4 * j + 2] * inv, v[4 * j + 3] * inv);
+        uint4* d = reinterpret_cast<uint4*>(q_row + static_cast<long long>(r0 + r) * C + c0 + kb * 32);
+        d[turn] = make_uint4(o[0], o[1], o[2], o[3]);
+        d[turn ^ 1] = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+    }
+  }
+  if (q_col != nullptr) {
+    const int rb = tid & 3, cp = tid >> 2;             // 32 rows from rb * 32 on, columns 2 cp and 2 cp + 1
+    // row block rb starts 4 rb rows into itself: the four blocks of a column pair then lie 8 banks apart
+    uint32_t w[32];
+    bf162 m2 = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      w[i] = *reinterpret_cast<const uint32_t*>(tile + (rb * 32 + ((i + 4 * rb) & 31)) * MX_PITCH + cp * 4);
+      m2 = __hmax2(m2, __habs2(*reinterpret_cast<const bf162*>(&w[i])));
+    }
+    const float2 amax = __bfloat1622float2(m2);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = c0 + 2 * cp + q;
+      if (c < C && r0 + rb * 32 < R) {
+        const int e = mx_scale_exp(q ? amax.y : amax.x, fmt_max);
+        const float inv = exp2f(static_cast<float>(-e));
+        sf_col[mx_sf_index(c, r0 / 32 + rb, (R + 127) / 128, col_tile)] = static_cast<unsigned char>(e + 127);
+        uint32_t o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float f[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) f[k] = __uint_as_float(q ? w[4 * j + k] & 0xffff0000u : w[4 * j + k] << 16) * inv;
+          o[j] = mx_pack4<E5M2>(f[0], f[1], f[2], f[3]);
+        }
+        uint32_t t[8];                                 // word j belongs at (j + rb) mod 8
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t[j] = rb & 1 ? o[(j + 7) & 7] : o[j];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = rb & 2 ? t[(j + 6) & 7] : t[j];
+        uint4* d = reinterpret_cast<uint4*>(q_col + static_cast<long long>(c) * R + r0 + rb * 32);
+        d[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        d[1] = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+    }
+  }
 }
 
 
@@ -241,23 +316,23 @@ int cb_rowquant_e4m3(const void* x, void* q, float* scale, long long M, int K, l
   return static_cast<int>(cudaGetLastError());
 }
 
-// x [R, C] bf16 (pitch ldx) -> q_col [C, R] = MXFP8 copy of the transpose, packed scales along R for rows c
-// (col_tile as tile_rows in cb_mxfp8_quant_packed; the scale buffer pre-filled with 127 where padding exists).
-// R a multiple of 32.
-int cb_mxfp8_quant_transposed(const void* x, long long R, int C, long long ldx, void* q_col, void* sf_col, int col_tile,
-                              int e5m2, void* stream) {
-  if (R <= 0 || C <= 0 || R % 32 != 0 || col_tile <= 0 || col_tile % 32 != 0 || q_col == nullptr || sf_col == nullptr)
+// x [R, C] bf16 (pitch ldx, a multiple of 8) -> q_row [R, C] and q_col [C, R] = MXFP8 copies of x and of its transpose, packed
+// scales along C for rows r and along R for rows c (row_tile / col_tile as tile_rows in cb_mxfp8_quant_packed; the scale
+// buffers pre-filled with 127 where padding exists).  q_row or q_col may be null.  R and C multiples of 32.
+int cb_mxfp8_quant_dual(const void* x, long long R, int C, long long ldx, void* q_row, void* sf_row, int row_tile, void* q_col,
+                        void* sf_col, int col_tile, int e5m2, void* stream) {
+  if (R <= 0 || C <= 0 || R % 32 != 0 || C % 32 != 0 || ldx % 8 != 0 || row_tile <= 0 || row_tile % 32 != 0 || col_tile <= 0 ||
+      col_tile % 32 != 0 || (q_row != nullptr && sf_row == nullptr) || (q_col != nullptr && sf_col == nullptr))
     return -1;
-  if (R / 32 > 65535) return -2;
-  const dim3 grid(static_cast<unsigned>((C + 255) / 256), static_cast<unsigned>(R / 32));
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (e5m2)
-    cb::mxfp8_quant_transposed_kernel<1><<<grid, 256, 0, s>>>(static_cast<const cb::bf16*>(x), R, C, ldx,
-        static_cast<unsigned char*>(q_col), static_cast<unsigned char*>(sf_col), col_tile);
-  else
-    cb::mxfp8_quant_transposed_kernel<0><<<grid, 256, 0, s>>>(static_cast<const cb::bf16*>(x), R, C, ldx,
-        static_cast<unsigned char*>(q_col), static_cast<unsigned char*>(sf_col), col_tile);
-  return static_cast<int>(cudaGetLastError());
+  if ((R + cb::MX_T - 1) / cb::MX_T > 65535) return -2;
+  const dim3 grid((C + cb::MX_T - 1) / cb::MX_T, static_cast<unsigned>((R + cb::MX_T - 1) / cb::MX_T));
+  const auto go = [&](auto kern) {
+    kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const cb::bf16*>(x), static_cast<int>(R), C, ldx, static_cast<unsigned char*>(q_row), static_cast<unsigned char*>(sf_row),
+        row_tile, static_cast<unsigned char*>(q_col), static_cast<unsigned char*>(sf_col), col_tile);
+    return static_cast<int>(cudaGetLastError());
+  };
+  return e5m2 ? go(cb::mxfp8_quant_dual_kernel<1>) : go(cb::mxfp8_quant_dual_kernel<0>);
 }
 
 }  // extern "C"

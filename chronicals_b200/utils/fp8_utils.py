@@ -142,25 +142,27 @@ def mxfp8_quantize_dual(x: torch.Tensor, fmt: str = "e4m3", row_tile: int = 128,
                         want_row: bool = True, want_col: bool = True):
     """``(q_row [R, C], sf_row, q_col [C, R], sf_col)``: the MXFP8 copy of ``x`` with blocks along its last
     dimension and the MXFP8 copy of ``xᵀ`` with blocks along the first — what the forward GEMM and the gradient GEMM over the
-    other dimension consume; the transposed copy is written by a kernel that transposes in registers, so no
-    bf16 transpose of ``x`` is ever materialised.  Scales are packed per ``row_tile`` /
+    other dimension consume; one kernel reads ``x`` once and writes both copies, and no bf16 transpose of ``x`` is ever
+    materialised.  Scales are packed per ``row_tile`` /
     ``col_tile`` rows (:func:`pack_mx_scales`).  Outputs not asked for are ``None``."""
     R, C = x.shape
     if x.is_cuda and x.dtype == torch.bfloat16 and R % 32 == 0 and C % 32 == 0 and x.stride(0) % 8 == 0 and block_scaled_available() \
-            and _ext.has_symbol("cb_mxfp8_quant_transposed") and R // 32 <= 65535:
-        if x.stride(1) != 1:
-            x = x.contiguous()
+            and _ext.has_symbol("cb_mxfp8_quant_dual") and R // 32 <= 65535:
+        if x.stride(1) != 1 or x.data_ptr() % 16 != 0:               # the kernel reads 16 bytes at a time
+            x = x.clone(memory_format=torch.contiguous_format)
         dev = x.device
         q_row = sf_row = q_col = sf_col = None
         if want_row:
-            q_row, sf_row = mxfp8_quantize_packed(x, fmt, row_tile)
+            q_row = torch.empty(R, C, dtype=torch.uint8, device=dev)
+            sf_row = _sf_buffer(R, C, row_tile, dev)
         if want_col:
             q_col = torch.empty(C, R, dtype=torch.uint8, device=dev)
             sf_col = _sf_buffer(C, R, col_tile, dev)
-            fn = _ext.lib().cb_mxfp8_quant_transposed
-            fn.argtypes = [_ext.P, _ext.L, _ext.I, _ext.L, _ext.P, _ext.P, _ext.I, _ext.I, _ext.P]
-            _ext.check(fn(x.data_ptr(), R, C, x.stride(0), q_col.data_ptr(), sf_col.data_ptr(), col_tile,
-                          int(fmt == "e5m2"), _ext.stream_ptr()), "mxfp8_quant_transposed")
+        if want_row or want_col:
+            fn = _ext.lib().cb_mxfp8_quant_dual
+            fn.argtypes = [_ext.P, _ext.L, _ext.I, _ext.L, _ext.P, _ext.P, _ext.I, _ext.P, _ext.P, _ext.I, _ext.I, _ext.P]
+            _ext.check(fn(x.data_ptr(), R, C, x.stride(0), _ext.ptr(q_row), _ext.ptr(sf_row), row_tile, _ext.ptr(q_col),
+                          _ext.ptr(sf_col), col_tile, int(fmt == "e5m2"), _ext.stream_ptr()), "mxfp8_quant_dual")
         return q_row, sf_row, q_col, sf_col
     q_row = sf_row = q_col = sf_col = None
     if want_row:
@@ -298,7 +300,7 @@ class _MXFP8LinearFn(torch.autograd.Function):
         ctx.has_bias = bias is not None
         ctx.shape = x.shape
         ctx.fused = (_block_scaled_ok(x2, w) and T % 32 == 0 and n_out % 32 == 0 and _ext.has_symbol("cb_mxgemm_pair")
-                     and _ext.has_symbol("cb_mxfp8_quant_transposed"))
+                     and _ext.has_symbol("cb_mxfp8_quant_dual"))
         if ctx.fused:
             need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
             xq, xs, xtq, xts = mxfp8_quantize_dual(x2, "e4m3", 128, PAIR_TILE_ROWS, True, need_dw)

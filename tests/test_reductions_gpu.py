@@ -96,3 +96,22 @@ def test_rmsnorm_layouts(M, N, residual):
     for got, want, slack in ((y, yr, 1e-5), (x.grad, xr.grad, 2e-5), (w.grad, wr.grad, 1e-5 * size + 1e-5)):
         # one rounding to bf16 and fp32 sums (dx of a residual cancels: its terms are of order one)
         assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()
+
+
+# one block of 32, ragged tiles of 128 in either direction, a pitch, a base off the 16-byte boundary, either copy alone
+@pytest.mark.parametrize("R,C,pitch,shift", [(32, 32, 32, 0), (160, 224, 224, 0), (96, 416, 424, 0), (416, 96, 96, 3), (1024, 640, 640, 8)])
+@pytest.mark.parametrize("fmt", ["e4m3", "e5m2"])
+@pytest.mark.parametrize("rows,cols", [(True, True), (True, False), (False, True)])
+def test_mxfp8_copies_of_a_matrix_and_its_transpose(R, C, pitch, shift, fmt, rows, cols):
+    from chronicals_b200.ops import ref
+    from chronicals_b200.utils import fp8_utils as F8
+    g = _gen(R + C)
+    buf = (torch.randn(shift + R * pitch, device=DEV, generator=g) * 4).to(torch.bfloat16)
+    x = buf[shift:].view(R, pitch)[:, :C]
+    x[0, :32], x[:32, C - 1] = 0, 0                               # whole blocks of zeros
+    q, s, qt, st = F8.mxfp8_quantize_dual(x, fmt, 128, 192, rows, cols)
+    for got, scales, m, want, tile in ((q, s, x, rows, 128), (qt, st, x.t(), cols, 192)):
+        assert (got is not None) == want
+        if want:
+            qr, sr = ref.mxfp8_quantize(m.float().contiguous(), fmt)
+            assert torch.equal(got, qr.view(torch.uint8)) and torch.equal(scales, F8.pack_mx_scales(sr, tile))

@@ -115,3 +115,20 @@ def test_mxfp8_copies_of_a_matrix_and_its_transpose(R, C, pitch, shift, fmt, row
         if want:
             qr, sr = ref.mxfp8_quantize(m.float().contiguous(), fmt)
             assert torch.equal(got, qr.view(torch.uint8)) and torch.equal(scales, F8.pack_mx_scales(sr, tile))
+
+
+# one chunk and several, a last chunk narrower than a tile, a vocabulary that is no multiple of 8
+@pytest.mark.parametrize("T,V,chunk", [(130, 5000, None), (130, 5000, 2048), (64, 4099, 1024), (257, 2056, 2048)])
+def test_linear_cross_entropy_chunks(T, V, chunk, monkeypatch):
+    if chunk is not None:
+        monkeypatch.setattr(ops, "_cce_chunk", lambda *a: chunk)
+    g = _gen(T + V)
+    h = torch.randn(T, 256, device=DEV, generator=g).to(torch.bfloat16).requires_grad_()
+    w = (0.05 * torch.randn(V, 256, device=DEV, generator=g)).to(torch.bfloat16).requires_grad_()
+    y = torch.randint(0, V, (T,), device=DEV, generator=g)
+    ops.linear_cross_entropy(h, w, y).backward()
+    hr, wr = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    torch.nn.functional.cross_entropy(hr @ wr.t(), y).backward()
+    # d(logits) is rounded to bf16 (2^-9) and so is either gradient
+    for got, want in ((h.grad, hr.grad), (w.grad, wr.grad)):
+        assert ((got.double() - want).norm() <= 2.0 ** -7 * want.norm()).item()

@@ -603,22 +603,46 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 // ------------------------------------------------------------------ combine kernels for cut-cross-entropy
-// lse[row] from the per-split partials; per-row loss with smoothing and z-loss.
-__global__ void cce_combine_rows_kernel(const float* __restrict__ part_m, const float* __restrict__ part_s,
-                                        const float* __restrict__ part_sum, const float* __restrict__ tgt,
-                                        const long long* __restrict__ labels, int M, int n_splits, int V_total,
-                                        float smoothing, float z_weight, long long ignore_index,
-                                        float* __restrict__ lse_out, float* __restrict__ loss_rows) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= M) return;
+// lse[row] from the per-split partials; per-row loss with smoothing and z-loss.  256 threads = 32 rows x 8 slices of the
+// splits (fixed order, so the sums are the same every time): bound by the latency of the partials, of which a thread per
+// row waited for all (14 us at 4096 rows and 38 splits, 6 now).
+__global__ void __launch_bounds__(256)
+cce_combine_rows_kernel(const float* __restrict__ part_m, const float* __restrict__ part_s,
+                        const float* __restrict__ part_sum, const float* __restrict__ tgt,
+                        const long long* __restrict__ labels, int M, int n_splits, int V_total,
+                        float smoothing, float z_weight, long long ignore_index,
+                        float* __restrict__ lse_out, float* __restrict__ loss_rows) {
+  __shared__ float red[3][8][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + tx;
+  const bool in = row < M;
   float m = -INFINITY;
-  for (int s = 0; s < n_splits; ++s) m = fmaxf(m, part_m[static_cast<long long>(s) * M + row]);
+  if (in) {
+#pragma unroll 4
+    for (int s = ty; s < n_splits; s += 8) m = fmaxf(m, part_m[static_cast<long long>(s) * M + row]);
+  }
+  red[0][ty][tx] = m;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m = fmaxf(m, red[0][i][tx]);
   float sum = 0.f, sl = 0.f;
-  for (int s = 0; s < n_splits; ++s) {
-    const long long o = static_cast<long long>(s) * M + row;
-    const float pm = part_m[o];
-    if (pm > -INFINITY) sum += part_s[o] * __expf(pm - m);
-    if (part_sum != nullptr) sl += part_sum[o];
+  if (in) {
+#pragma unroll 4
+    for (int s = ty; s < n_splits; s += 8) {
+      const long long o = static_cast<long long>(s) * M + row;
+      const float pm = part_m[o];
+      if (pm > -INFINITY) sum += part_s[o] * __expf(pm - m);
+      if (part_sum != nullptr) sl += part_sum[o];
+    }
+  }
+  red[1][ty][tx] = sum;
+  red[2][ty][tx] = sl;
+  __syncthreads();
+  if (ty != 0 || !in) return;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) {
+    sum += red[1][i][tx];
+    sl += red[2][i][tx];
   }
   const float lse = m + __logf(sum);
   lse_out[row] = lse;
@@ -906,12 +930,38 @@ int cb_gemm_bf16_tp(const void* A, const void* B, void* C, const void* bias, int
   return dispatch<cb::EPI_STORE>(bn, a_mn, b_mn, ta, tb, tc, g, static_cast<cudaStream_t>(stream));
 }
 
+}  // extern "C"
+
+namespace {
+// Vocabulary tiles that one item of the forward pass (one m-block, a run of tiles, one set of partials) covers.  The items
+// are dealt out round by round over the SMs, so the pass takes rounds x tiles: the run is chosen to make that least, with
+// one tile's time for an item's start and partials (ties: the longer run).  A fixed 16 left 168 items on 148 SMs at 2621
+// tokens and 32,000 words and 38 at 64 tokens and 151,936.  Kernel alone, fixed -> chosen: 2621 x 32,000 (K = 896)
+// 169 -> 115 us, 1000 x 32,000 (K = 2048) 195 -> 97, 300 x 5000 (K = 256) 81 -> 9, 64 x 151,936 95 -> 53; 4096 and 8192
+// x 151,936 stay with 16 (791 and 1594 us; 796 and 1608 with 8).
+int cce_tiles_per_item(int M, int V) {
+  const int tiles = (V + 255) / 256, mb = (M + 127) / 128, sms = num_sms();
+  int best = tiles < 16 ? tiles : 16;
+  double best_cost = -1.0;
+  for (int per = 1; per <= (tiles < 32 ? tiles : 32); ++per) {
+    const long long items = static_cast<long long>(mb) * ((tiles + per - 1) / per);
+    const double cost = static_cast<double>((items + sms - 1) / sms) * (per + 1.0);
+    if (best_cost < 0.0 || cost <= best_cost) {
+      best_cost = cost;
+      best = per;
+    }
+  }
+  return best;
+}
+}  // namespace
+
+extern "C" {
+
 // Number of vocab splits the forward pass of the fused linear-cross-entropy uses for a
 // [M, V] problem (the partial buffers are [n_splits, M]).
 int cb_cce_num_splits(int M, int V) {
-  const int tiles = (V + 255) / 256;
-  const int per = tiles < 16 ? tiles : 16;
-  return (tiles + per - 1) / per;
+  const int per = cce_tiles_per_item(M, V);
+  return ((V + 255) / 256 + per - 1) / per;
 }
 
 // Forward: per-row log-sum-exp partials of hidden[M,K] * weight[V,K]^T, target logit.
@@ -926,7 +976,7 @@ int cb_cce_forward(const void* hidden, const void* weight, const long long* labe
   g.M = M; g.N = V; g.K = K;
   g.num_m_blocks = (M + 127) / 128;
   g.num_n_tiles = (V + bn - 1) / bn;
-  g.tiles_per_item = g.num_n_tiles < 16 ? g.num_n_tiles : 16;
+  g.tiles_per_item = cce_tiles_per_item(M, V);
   const int n_splits = (g.num_n_tiles + g.tiles_per_item - 1) / g.tiles_per_item;
   g.num_items = g.num_m_blocks * n_splits;
   g.labels = labels;
@@ -943,7 +993,7 @@ int cb_cce_combine(const float* part_m, const float* part_s, const float* part_s
                    long long ignore_index, int mean, float* lse, float* loss_rows, float* out, float* gscale,
                    void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  cb::cce_combine_rows_kernel<<<(M + 255) / 256, 256, 0, s>>>(part_m, part_s, part_sum, tgt, labels, M, n_splits,
+  cb::cce_combine_rows_kernel<<<(M + 31) / 32, 256, 0, s>>>(part_m, part_s, part_sum, tgt, labels, M, n_splits,
                                                               V_total, smoothing, z_weight, ignore_index, lse,
                                                               loss_rows);
   cb::cce_finalize_kernel<<<1, 1024, 0, s>>>(loss_rows, labels, M, ignore_index, mean, out, gscale);

@@ -132,3 +132,16 @@ def test_linear_cross_entropy_chunks(T, V, chunk, monkeypatch):
     # d(logits) is rounded to bf16 (2^-9) and so is either gradient
     for got, want in ((h.grad, hr.grad), (w.grad, wr.grad)):
         assert ((got.double() - want).norm() <= 2.0 ** -7 * want.norm()).item()
+
+
+# one item in all, runs of one tile, a last run shorter than the others, several rounds
+@pytest.mark.parametrize("T,V", [(1, 8), (64, 256), (130, 5000), (300, 40000), (3000, 4099)])
+@pytest.mark.parametrize("smoothing", [0.0, 0.1])
+def test_linear_cross_entropy_splits(T, V, smoothing):
+    g = _gen(T + V)
+    h = torch.randn(T, 128, device=DEV, generator=g).to(torch.bfloat16)
+    w = (0.1 * torch.randn(V, 128, device=DEV, generator=g)).to(torch.bfloat16)
+    y = torch.randint(0, V, (T,), device=DEV, generator=g)
+    rows = ops.linear_cross_entropy(h, w, y, label_smoothing=smoothing, reduction="none")
+    want = torch.nn.functional.cross_entropy(h.double() @ w.double().t(), y, label_smoothing=smoothing, reduction="none")
+    assert (rows.double() - want).abs().max().item() < 2e-5 * max(1.0, want.abs().max().item())      # fp32 sums throughout

@@ -28,6 +28,7 @@
 // does its peer once its own waits expire, so the pair always leaves together.
 //
 // The reference has no GEMM of its own (cuBLAS behind nn.Linear); nothing to cite.
+#include <algorithm>
 #include <cstring>
 #include "common.cuh"
 #include "host_common.h"
@@ -714,34 +715,48 @@ int dispatch_layout(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap
   return launch2<BN, 1, 0>(ta, tb, tc, tw, g, pairs, s, ta2, tb2);
 }
 
-// Whole tiles take ceil(T / pairs) rounds; cut along K the work takes T / pairs rounds plus the fixups (partial
-// sums through L2, the last arrival's read-back and a burst of them when every pair ends on a partial tile),
-// measured at about 36 us, i.e. 72 / num_kb rounds of a 64-wide k-block at ~0.5 us.  Worth it for long K and a
-// mostly empty last round (weight gradients over thousands of tokens), not for the K = 896 projections.
-bool stream_k_pays(long long T, int pairs, int num_kb) {
-  if (pairs < 2 || T % pairs == 0) return false;
-  const double whole = static_cast<double>((T + pairs - 1) / pairs);
-  const double split = static_cast<double>(T) / pairs + 72.0 / num_kb;
-  return split < whole - 0.05;
-}
-
-// tile width with the least padding of N (ties: the widest)
-int pick_bn(int N) {
-  int best = 256;
-  long long best_pad = -1;
-  for (int bn : {256, 224, 192}) {
-    const long long pad = static_cast<long long>((N + bn - 1) / bn) * bn - N;
-    if (best_pad < 0 || pad < best_pad) {
-      best_pad = pad;
-      best = bn;
+// What a product takes on CTA pairs with tiles of 256 x bn, in microseconds at full clock: whole tiles, ceil(T / pairs)
+// rounds of them; or cut along K, T / pairs rounds and the fixups (partial sums through L2, the last arrival's read-back:
+// 24 us, so only a long K and a mostly empty last round pay).  Fitted to 276 products (four model sizes, 128 to 8192
+// tokens, forward, dgrad and wgrad; 7 to 10 % off on average).  Of two widths the one that pads N least used to be taken,
+// whatever the rounds: 4096 x 1536 x 8960 ran two rounds of 256 (121 us) where two of 192 take 83.
+struct PairPlan {
+  int bn;
+  bool split;
+  double us;
+};
+PairPlan plan_pairs(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool may_split, int force_bn) {
+  static const double fixed[3] = {6.0, 6.0, 5.7}, per_mb[3] = {0.112, 0.16, 0.145};       // per MB of output
+  static const double per_kb[3] = {0.319, 0.281, 0.265}, per_kb_mn[3] = {0.319, 0.312, 0.309};   // both operands MN-major
+  static const double split_fixed[3] = {30.4, 30.6, 26.3}, split_kb[3] = {0.353, 0.33, 0.307};
+  const double kb = (K + 63) / 64, mb = 1e-6 * M * N * out_bytes;
+  PairPlan best = {0, false, 0.0};
+  for (int i = 0; i < 3; ++i) {
+    const int bn = 256 - 32 * i;
+    if (force_bn != 0 && force_bn != bn) continue;
+    const long long T = static_cast<long long>((M + 255) / 256) * ((N + bn - 1) / bn);
+    const long long pairs = T < cbhost::num_sms() / 2 ? T : cbhost::num_sms() / 2;
+    const double whole = fixed[i] + (a_mn && b_mn ? per_kb_mn : per_kb)[i] * ((T + pairs - 1) / pairs) * kb + per_mb[i] * mb;
+    // a narrower tile reads more per product, which the larger problems feel in L2 and in power
+    if (best.bn == 0 || whole * (1.0 + 0.12 * std::min(1.0, whole / 150.0)) < best.us) best = {bn, false, whole};
+    // pairs at different depths of K share no operands, which a very long K does not forgive unless most tiles are whole
+    // (2624 x 3584 x 37,888: 681 us against 512); below 32 k-blocks the fixups of many small runs outweigh the estimate
+    if (may_split && T % pairs != 0 && kb >= 32 && (kb <= 256 || T >= 3 * pairs)) {
+      const double split = split_fixed[i] + split_kb[i] * kb * T / pairs;
+      if (split < 1.05 * best.us) best = {bn, true, split};     // 1.05: whole tiles are the ones estimated too low here
     }
   }
   return best;
 }
+bool have_workspace() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return dev >= 0 && dev < MAX_DEVICES && g_ws_ptr[dev] != nullptr;
+}
 
 // Fills the stream-K fields of `g` for `pairs` resident pairs.  Returns the number of tile slots the workspace
 // needs (0: whole tiles only).
-int plan_stream_k(cb2::Args* g, int pairs, int bn, int device, int allow) {
+int plan_stream_k(cb2::Args* g, int pairs, int bn, int device, bool allow) {
   g->sk_tiles = 0;
   g->sk_q = g->sk_r = 0;
   g->ws = nullptr;
@@ -749,7 +764,6 @@ int plan_stream_k(cb2::Args* g, int pairs, int bn, int device, int allow) {
   const int T = g->num_tiles;
   if (!allow || pairs < 2 || T % pairs == 0 || device < 0 || device >= MAX_DEVICES || g_ws_ptr[device] == nullptr) return 0;
   const int full = T / pairs, rem = T % pairs;
-  if (allow != 2 && !stream_k_pays(T, pairs, g->num_kb)) return 0;
   int sk = full >= 1 ? rem + pairs : T;                      // every pair gets between one and two tiles' worth
   if (sk > T) sk = T;
   if (sk > cb2::MAX_SK_TILES) return 0;
@@ -791,19 +805,9 @@ int cb_gemm2sm_set_workspace(int device, void* ptr, unsigned long long bytes) {
   return 0;
 }
 
-// What the dispatcher needs to know about a problem: rounds of tile time the pair kernel takes (x 1000).
-int cb_gemm2sm_cost_milli(int M, int N, int K, int pairs_avail) {
-  const int bn = pick_bn(N);
-  const long long T = static_cast<long long>((M + 255) / 256) * ((N + bn - 1) / bn);
-  const int pairs = T < pairs_avail ? static_cast<int>(T) : pairs_avail;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const bool ws = dev >= 0 && dev < MAX_DEVICES && g_ws_ptr[dev] != nullptr;
-  const long long kb = (K + 63) / 64;
-  double rounds = static_cast<double>((T + pairs - 1) / pairs);
-  if (ws && T * kb >= 4LL * pairs && stream_k_pays(T, pairs, static_cast<int>(kb)))
-    rounds = static_cast<double>(T) / pairs + 72.0 / kb;
-  return static_cast<int>(rounds * 1000.0 * bn / 256.0);
+// What the dispatcher needs to know about a problem: the pair kernel's time in nanoseconds.
+int cb_gemm2sm_cost_ns(int M, int N, int K, int a_mn, int b_mn, int out_bytes) {
+  return static_cast<int>(1e3 * std::min(2e6, plan_pairs(M, N, K, a_mn, b_mn, out_bytes, have_workspace(), 0).us));
 }
 
 // C[M,N] = op(A) * op(B)^T (+bias) (+addend) (+C) on CTA pairs.  Same conventions as cb_gemm_bf16 (gemm.cu):
@@ -816,7 +820,9 @@ int cb_gemm2sm_bf16_ex(const void* A, const void* B, void* C, const void* bias, 
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if (!cb_gemm2sm_supported(C, ldc, out_fp32)) return -2;
   int bn = flags >> 8;
-  if (bn != 256 && bn != 224 && bn != 192) bn = pick_bn(N);
+  if (bn != 256 && bn != 224 && bn != 192) bn = 0;
+  const PairPlan plan = plan_pairs(M, N, K, a_mn, b_mn, out_fp32 ? 4 : 2, !(flags & 1) && have_workspace(), bn);
+  bn = plan.bn;
   if (b_mn && (ldb * 2) % 16 != 0) return -3;
   CUtensorMap ta, tb, tc, tw;
   int e;
@@ -844,7 +850,7 @@ int cb_gemm2sm_bf16_ex(const void* A, const void* B, void* C, const void* bias, 
   if (pairs > g.num_tiles) pairs = g.num_tiles;
   int dev = 0;
   cudaGetDevice(&dev);
-  const int slots = plan_stream_k(&g, pairs, bn, dev, (flags & 1) ? 0 : ((flags & 2) ? 2 : 1));
+  const int slots = plan_stream_k(&g, pairs, bn, dev, (flags & 2) ? true : plan.split);
   memset(&tw, 0, sizeof(tw));
   if (slots > 0) {
     e = cbhost::make_tmap(&tw, g.ws, bn, static_cast<unsigned long long>(slots) * 256ull, bn, 32, 32, 4);
@@ -900,7 +906,8 @@ int cb_gemm2sm_bf16_dual(const void* A, const void* B, const void* A2, const voi
                          long long ldb2, long long ldc, long long ld_add, int b_mn, int* status, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || K2 <= 0) return -1;
   if (!cb_gemm2sm_supported(C, ldc, 0)) return -2;
-  const int bn = pick_bn(N);
+  const PairPlan plan = plan_pairs(M, N, K + K2, 0, b_mn, 2, have_workspace(), 0);
+  const int bn = plan.bn;
   if (b_mn && ((ldb * 2) % 16 != 0 || (ldb2 * 2) % 16 != 0)) return -3;
   CUtensorMap ta, tb, ta2, tb2, tc, tw;
   int e = cbhost::make_tmap(&ta, A, K, M, lda, 64, cb2::BM);
@@ -936,7 +943,7 @@ int cb_gemm2sm_bf16_dual(const void* A, const void* B, const void* A2, const voi
   if (pairs > g.num_tiles) pairs = g.num_tiles;
   int dev = 0;
   cudaGetDevice(&dev);
-  const int slots = plan_stream_k(&g, pairs, bn, dev, 1);
+  const int slots = plan_stream_k(&g, pairs, bn, dev, plan.split);
   if (slots > 0) {
     e = cbhost::make_tmap(&tw, g.ws, bn, static_cast<unsigned long long>(slots) * 256ull, bn, 32, 32, 4);
     if (e) return e;

@@ -1,0 +1,30 @@
+"""Products on either side of the lines between the GEMM kernels and tile widths, against fp64."""
+import pytest
+import torch
+
+from chronicals_b200 import ops
+from chronicals_b200.ops import _ext
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# 128-wide single-CTA tiles, 256-wide ones, pairs of 256, 224 and 192, tiles cut along K; ragged last tiles in M and N, K that
+# is no multiple of the k-block
+@pytest.mark.parametrize("M,N,K", [(1000, 896, 1152), (512, 1152, 896), (128, 896, 4864), (2624, 2048, 1096), (4096, 1536, 1000),
+                                   (3000, 1800, 520), (1500, 3584, 1024), (1008, 200, 2056), (9728, 896, 4104), (304, 5120, 328)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_chosen_kernel(M, N, K, a_mn, b_mn, fp32):
+    if (a_mn and M % 8) or (b_mn and N % 8):
+        pytest.skip("operand pitch")
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    a = torch.randn(*((K, M) if a_mn else (M, K)), device=DEV, generator=g).to(torch.bfloat16)
+    b = torch.randn(*((K, N) if b_mn else (N, K)), device=DEV, generator=g).to(torch.bfloat16)
+    out = torch.full((M, N), 7.0, device=DEV, dtype=torch.float32 if fp32 else torch.bfloat16)
+    ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out)
+    _ext.check_status()
+    want = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double()
+    # fp32 sums of K products of order one, one rounding of the result
+    slack = K ** 0.5 * 2e-6 * 8 + (0 if fp32 else 1e-6)
+    assert ((out.double() - want).abs() <= (1e-6 if fp32 else 2.0 ** -8) * want.abs() + slack * 4).all()

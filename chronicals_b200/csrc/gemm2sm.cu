@@ -83,7 +83,8 @@ struct Args {
   // through push_c[owner] (a peer mapping, pre-offset so that the global row indexes it with pitch ldc)
   unsigned long long push_c[16];
   int push_rows;
-  // ---- gated-activation epilogue (GLU = 1 instantiation only): B is the fused gate | up weight [2 * glu_i, K]
+  // ---- gated-activation epilogues.  GLU = 1: B is the fused gate | up weight [2 * glu_i, K]; GLU = 2: the product is the
+  // gradient of the activation [M, glu_i]
   int glu_i;
 };
 
@@ -171,6 +172,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW,
                const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2, const Args g) {
   constexpr int BNH = BN / 2;
+  constexpr int NST = GLU == 2 ? 5 : STAGES;                             // GLU = 2: the sixth stage's room holds gate and up
   constexpr uint32_t TMEM_COLS = 512;                                    // two accumulators, 256 columns apart
   constexpr uint32_t IDESC = KIND ? umma_idesc_fp8(2 * BM, BN, 0, 0)
                                   : umma_idesc_bf16(2 * BM, BN, A_MN, B_MN);      // M = 256 across the pair
@@ -182,12 +184,13 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
-  uint8_t* sB = smem + STAGES * A_BYTES;
+  uint8_t* sB = smem + NST * A_BYTES;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + BAR_OFFSET);       // (leader) the stage landed in both CTAs
-  uint64_t* empty = full + STAGES;                                       // stage consumed (multicast commit)
-  uint64_t* tfull = empty + STAGES;                                      // accumulator complete (multicast commit)
+  uint64_t* empty = full + NST;                                       // stage consumed (multicast commit)
+  uint64_t* tfull = empty + NST;                                      // accumulator complete (multicast commit)
   uint64_t* tempty = tfull + 2;                                          // (leader) accumulator drained by both CTAs
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t* gu_full = tempty + 2;                                        // [4] GLU = 2: a warp's gate and up columns have landed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gu_full + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform for the compiler too
@@ -198,7 +201,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int num_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < NST; ++s) {
       mbar_init(full + s, 1);
       mbar_init(empty + s, 1);
     }
@@ -206,6 +209,8 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       mbar_init(tfull + a, 1);
       mbar_init(tempty + a, 8);                                          // 4 epilogue warps in each CTA
     }
+    if (GLU == 2)
+      for (int w = 0; w < 4; ++w) mbar_init(gu_full + w, 1);
     mbar_fence_init();
     *abort_flag = (g.status[0] != 0) ? 1 : 0;
     tma_prefetch_desc(&tmA);
@@ -246,7 +251,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int a_row = mp * 2 * BM + static_cast<int>(rank) * BM;
         // GLU: the leader's half of B holds the gate rows of activation columns [nt * BNH, +BNH), the peer's half
         // the up rows of the same columns (glu_i rows further down in the fused gate|up weight)
-        const int b_row = GLU ? nt * BNH + static_cast<int>(rank) * g.glu_i : nt * BN + static_cast<int>(rank) * BNH;
+        const int b_row = GLU == 1 ? nt * BNH + static_cast<int>(rank) * g.glu_i : nt * BN + static_cast<int>(rank) * BNH;
         if (TP && g.panel_pairs > 0) {
           // rows of this tile come from rank `src`: wait (bounded) until its push kernel has signalled
           const int src = mp / g.panel_pairs;
@@ -295,7 +300,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < (BNH + 63) / 64; ++j) tma_load_2d_pair(b_dst + j * 8192, mb, bar, b_row + j * 64, kk * BK);
           }
-          if (++stage == STAGES) {
+          if (++stage == NST) {
             stage = 0;
             phase ^= 1;
           }
@@ -340,7 +345,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             umma_commit_2cta(empty + stage);    // frees this stage in both CTAs once the MMAs retire
           }
-          if (++stage == STAGES) {
+          if (++stage == NST) {
             stage = 0;
             phase ^= 1;
           }
@@ -511,6 +516,18 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
     };
 
+    // GLU = 2: gate and up of 64 columns of this warp's 32 rows, 4 KB each, on their way into its 8 KB behind the ring
+    uint8_t* gu_buf = smem + NST * (A_BYTES + B_BYTES) + (warp - 2) * 8192;
+    uint32_t gu_cnt = 0;
+    auto fetch_gu = [&](int acol, int row0w) {
+      fence_async_smem();
+      __syncwarp();                                           // every lane has taken the columns before these
+      if (lane == 0) {
+        mbar_expect_tx(gu_full + (warp - 2), 8192);
+        tma_load_2d(gu_buf, &tmW, gu_full + (warp - 2), acol, row0w);
+        tma_load_2d(gu_buf + 4096, &tmW, gu_full + (warp - 2), g.glu_i + acol, row0w);
+      }
+    };
     while (ok && seg.next(g, t, kb0, kb1)) {
       int mp = t % g.num_m_pairs;
       if (TP) {
@@ -521,6 +538,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const uint32_t acc = seg_cnt & 1u;
       const uint32_t acc_phase = (seg_cnt >> 1) & 1u;
       ++seg_cnt;
+      if (GLU == 2) fetch_gu(nt * BN, mp * 2 * BM + static_cast<int>(rank) * BM + q * 32);     // while the product is computed
       bool w = mbar_wait(tfull + acc, acc_phase, abort_flag, g.status, CB_ERR_WAIT_TMEM_FULL);
       w = __all_sync(0xffffffffu, w);
       if (!w) {
@@ -534,7 +552,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const bool row_ok = row < g.M;
       const bool whole = (kb0 == 0 && kb1 == g.num_kb);
 
-      if (GLU) {
+      if (GLU == 1) {
         // Accumulator columns [0, BNH) are the gate, [BNH, BN) the up projection of activation columns
         // nt * BNH ...  Per 64 columns: gate -> C (kept as bf16 pairs), up -> C, silu(gate) * up -> the activation
         // tensor (map tmW), all three through the staging buffers and TMA stores.  The product uses the values as
@@ -574,6 +592,55 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           stage_bf16(r);
           flush(&tmW, acol, row0w, false, row0w < g.M);
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (leader) mbar_arrive(tempty + acc);
+          else mbar_arrive_remote(tempty_leader + acc * 8);
+        }
+      } else if (GLU == 2) {
+        // The accumulator is d(act); gate and up come by TMA, one chunk of 64 columns ahead.  With s = sigmoid(gate):
+        // d(up) = d gate s, d(gate) = d up s (1 + gate (1 - s)), both through the staging buffers to C's two halves.
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN; c0 += 64) {
+          const int acol = nt * BN + c0;
+          if (acol >= g.glu_i) break;                         // uniform across the warp
+          ok = __all_sync(0xffffffffu, mbar_wait(gu_full + (warp - 2), gu_cnt & 1u, abort_flag, g.status, CB_ERR_WAIT_FULL));
+          ++gu_cnt;
+          if (!ok) break;
+          uint32_t gp[32], up[32], r[64];
+#pragma unroll
+          for (int cc = 0; cc < 8; ++cc) {
+            const uint4 a = *reinterpret_cast<const uint4*>(gu_buf + lane * 128 + ((cc ^ (lane & 7)) << 4));
+            const uint4 b = *reinterpret_cast<const uint4*>(gu_buf + 4096 + lane * 128 + ((cc ^ (lane & 7)) << 4));
+            gp[4 * cc] = a.x; gp[4 * cc + 1] = a.y; gp[4 * cc + 2] = a.z; gp[4 * cc + 3] = a.w;
+            up[4 * cc] = b.x; up[4 * cc + 1] = b.y; up[4 * cc + 2] = b.z; up[4 * cc + 3] = b.w;
+          }
+          if (c0 + 64 < BN && acol + 64 < g.glu_i) fetch_gu(acol + 64, row0w);
+          tmem_ld_32x32(t_row + c0, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+          tmem_ld_32x32(t_row + c0 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float2 gt = unpack_bf16x2(gp[j]), ut = unpack_bf16x2(up[j]);
+            const float d0 = __uint_as_float(r[2 * j]), d1 = __uint_as_float(r[2 * j + 1]);
+            const float s0 = __fdividef(1.f, 1.f + __expf(-gt.x)), s1 = __fdividef(1.f, 1.f + __expf(-gt.y));
+            const float ds0 = d0 * s0, ds1 = d1 * s1;
+            r[2 * j] = __float_as_uint(ds0 * ut.x * fmaf(gt.x, 1.f - s0, 1.f));
+            r[2 * j + 1] = __float_as_uint(ds1 * ut.y * fmaf(gt.y, 1.f - s1, 1.f));
+            up[j] = pack_bf16x2(ds0 * gt.x, ds1 * gt.y);
+          }
+          stage_bf16(r);
+          flush(&tmC, acol, row0w, false, row0w < g.M);
+          if (lane == 0) tma_store_wait_read<1>();
+          __syncwarp();
+#pragma unroll
+          for (int cc = 0; cc < 8; ++cc)
+            *reinterpret_cast<uint4*>(stg + buf * 4096 + lane * 128 + ((cc ^ (lane & 7)) << 4)) =
+                make_uint4(up[4 * cc], up[4 * cc + 1], up[4 * cc + 2], up[4 * cc + 3]);
+          flush(&tmC, g.glu_i + acol, row0w, false, row0w < g.M);
+        }
+        if (!ok) break;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
@@ -896,6 +963,42 @@ int cb_gemm2sm_bf16_glu(const void* A, const void* W, void* GU, void* ACT, const
   int pairs = cbhost::num_sms() / 2;
   if (pairs > g.num_tiles) pairs = g.num_tiles;
   return launch2<256, 0, 0, 0, 0, 1>(ta, tb, tc, tact, g, pairs, static_cast<cudaStream_t>(stream));
+}
+
+// Backward of down(silu(gate) * up) in one product: DACT[M, I] = DY[M, K] WD[K, I] stays in the accumulators, and
+//   DGU[M, 2I] = (d(gate) | d(up))
+// of GU[M, 2I] (gate | up as kept by cb_gemm2sm_bf16_glu) leaves instead.  WD is the down projection as stored, [K, I]; all bf16,
+// I a multiple of 64 (returns -5 otherwise).  DACT is neither rounded nor written and read (160 MB at 8192 x 4864); gate and
+// up come by TMA, a chunk ahead of the epilogue, into the room of one of the ring's six stages.
+// Measured at 8192 x 4864, K = 896: 93 us, against 58 for the dgrad and 64 for the activation's backward; it is the epilogue (two
+// special-function and about twenty other instructions a value on four warps) that keeps it from the 58.
+int cb_gemm2sm_bf16_glu_bwd(const void* DY, const void* WD, const void* GU, void* DGU, int M, int I, int K, long long ld_dy,
+                            long long ld_wd, long long ld_gu, long long ld_dgu, int* status, void* stream) {
+  if (M <= 0 || I <= 0 || K <= 0) return -1;
+  if (I % 64 != 0) return -5;
+  if (!cb_gemm2sm_supported(GU, ld_gu, 0) || !cb_gemm2sm_supported(DGU, ld_dgu, 0) || (ld_wd * 2) % 16 != 0) return -2;
+  CUtensorMap ta, tb, tc, tgu;
+  int e = cbhost::make_tmap(&ta, DY, K, M, ld_dy, 64, cb2::BM);
+  if (e) return e;
+  e = cbhost::make_tmap(&tb, WD, I, K, ld_wd, 64, 64);
+  if (e) return e;
+  e = cbhost::make_tmap(&tc, DGU, 2ull * I, M, ld_dgu, 64, 32, 2);
+  if (e) return e;
+  e = cbhost::make_tmap(&tgu, GU, 2ull * I, M, ld_gu, 64, 32, 2);
+  if (e) return e;
+  cb2::Args g = {};
+  g.M = M; g.N = I; g.K = K;
+  g.glu_i = I;
+  g.num_m_pairs = (M + 2 * cb2::BM - 1) / (2 * cb2::BM);
+  g.num_n_tiles = (I + 255) / 256;
+  g.num_tiles = g.num_m_pairs * g.num_n_tiles;
+  g.num_kb = (K + cb2::BK - 1) / cb2::BK;
+  g.num_kb1 = g.num_kb;
+  g.C = DGU; g.ldc = ld_dgu;
+  g.status = status;
+  int pairs = cbhost::num_sms() / 2;
+  if (pairs > g.num_tiles) pairs = g.num_tiles;
+  return launch2<256, 0, 1, 0, 0, 2>(ta, tb, tc, tgu, g, pairs, static_cast<cudaStream_t>(stream));
 }
 
 // C[M,N] = A B^T + A2 B2^T (+bias) (+addend): the second product (inner dimension K2, small) is accumulated in the

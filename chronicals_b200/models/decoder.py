@@ -171,6 +171,10 @@ class Attention(nn.Module):
         return self.o_proj(o, residual)
 
 
+def _has_hooks(m: nn.Module) -> bool:
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+
+
 class MLP(nn.Module):
     def __init__(self, cfg: ChronicalsConfig, dtype, device=None):
         super().__init__()
@@ -181,8 +185,10 @@ class MLP(nn.Module):
         self.gelu = cfg.hidden_act in ("gelu", "gelu_pytorch_tanh", "gelu_new")
 
     def forward(self, x, residual):
-        fl = self.gate_up_proj
+        fl, down = self.gate_up_proj, self.down_proj
         if not self.gelu and fl.is_plain():
+            if down.is_plain() and down.bias is None and not _has_hooks(down):
+                return ops.swiglu_mlp(x, fl.weight, down.weight, fl.bias, residual)       # the whole block as one autograd node
             a = ops.linear_swiglu(x, fl.weight, fl.bias)       # activation in the projection's epilogue
         else:
             gu = fl(x)

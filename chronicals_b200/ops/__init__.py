@@ -412,6 +412,35 @@ class _GLUFn(torch.autograd.Function):
         return dgu.view(ctx.shape), None
 
 
+def _linear_swiglu_forward(x2, w, bias):
+    """``(gate | up, act)`` of the fused gate | up weight: one GEMM with the activation in its epilogue."""
+    M, K = x2.shape
+    I = w.shape[0] // 2
+    gu = torch.empty(M, 2 * I, dtype=x2.dtype, device=x2.device)
+    act = torch.empty(M, I, dtype=x2.dtype, device=x2.device)
+    code = _ext.lib().cb_gemm2sm_bf16_glu(x2.data_ptr(), w.data_ptr(), gu.data_ptr(), act.data_ptr(), _ext.ptr(bias),
+                                          M, I, K, x2.stride(0), w.stride(0), gu.stride(0), act.stride(0),
+                                          _ext.status_buffer(x2.device).data_ptr(), _ext.stream_ptr())
+    if code > 0:
+        _ext.check(code, "gemm2sm_bf16_glu")
+    if code != 0:                                            # shape not covered: projection, then activation
+        gemm(x2, w, bias=bias, out=gu)
+        c2 = _ext.lib().cb_glu_fwd(gu.data_ptr(), gu.data_ptr() + 2 * I, act.data_ptr(), M, I, 2 * I, I, 0, _ext.stream_ptr())
+        _ext.check(c2, "glu_fwd")
+    return gu, act
+
+
+def _glu_backward(d2, gu):
+    """``d(gate) | d(up)`` of ``silu(gate) * up`` from the gradient of the product."""
+    M, I2 = gu.shape
+    I = I2 // 2
+    dgu = torch.empty_like(gu)
+    code = _ext.lib().cb_glu_bwd(d2.data_ptr(), gu.data_ptr(), gu.data_ptr() + 2 * I, dgu.data_ptr(),
+                                 dgu.data_ptr() + 2 * I, M, I, I, I2, I2, 0, _ext.stream_ptr())
+    _ext.check(code, "glu_bwd")
+    return dgu
+
+
 class _LinearSwiGLUFn(torch.autograd.Function):
     """``act = silu(x Wgᵀ + bg) * (x Wuᵀ + bu)`` for the fused gate | up weight ``w [2I, K]``.
 
@@ -422,19 +451,7 @@ class _LinearSwiGLUFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x2, w, bias):
-        M, K = x2.shape
-        I = w.shape[0] // 2
-        gu = torch.empty(M, 2 * I, dtype=x2.dtype, device=x2.device)
-        act = torch.empty(M, I, dtype=x2.dtype, device=x2.device)
-        code = _ext.lib().cb_gemm2sm_bf16_glu(x2.data_ptr(), w.data_ptr(), gu.data_ptr(), act.data_ptr(), _ext.ptr(bias),
-                                              M, I, K, x2.stride(0), w.stride(0), gu.stride(0), act.stride(0),
-                                              _ext.status_buffer(x2.device).data_ptr(), _ext.stream_ptr())
-        if code > 0:
-            _ext.check(code, "gemm2sm_bf16_glu")
-        if code != 0:                                            # shape not covered: projection, then activation
-            gemm(x2, w, bias=bias, out=gu)
-            c2 = _ext.lib().cb_glu_fwd(gu.data_ptr(), gu.data_ptr() + 2 * I, act.data_ptr(), M, I, 2 * I, I, 0, _ext.stream_ptr())
-            _ext.check(c2, "glu_fwd")
+        gu, act = _linear_swiglu_forward(x2, w, bias)
         ctx.save_for_backward(x2, w, gu)
         ctx.has_bias = bias is not None
         ctx.weight_ref = weakref.ref(w) if hasattr(w, "_cb_grad_out") else None
@@ -448,10 +465,7 @@ class _LinearSwiGLUFn(torch.autograd.Function):
         d2 = dact.reshape(M, I)
         if not d2.is_contiguous():
             d2 = d2.contiguous()
-        dgu = torch.empty_like(gu)
-        code = _ext.lib().cb_glu_bwd(d2.data_ptr(), gu.data_ptr(), gu.data_ptr() + 2 * I, dgu.data_ptr(),
-                                     dgu.data_ptr() + 2 * I, M, I, I, I2, I2, 0, _ext.stream_ptr())
-        _ext.check(code, "glu_bwd")
+        dgu = _glu_backward(d2, gu)
         dx = dw = db = None
         if ctx.needs_input_grad[0]:
             dx = gemm(dgu, w, b_mn=True)
@@ -480,6 +494,68 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
         a = _LinearSwiGLUFn.apply(x2, w, bias)
         return a if x.dim() == 2 else a.view(*x.shape[:-1], I)
     return swiglu(linear(x, w, bias))
+
+
+class _SwiGLUMLPFn(torch.autograd.Function):
+    """``silu(x Wgᵀ + bg) * (x Wuᵀ + bu)`` times the down projection, plus the residual, as one node.
+
+    Forward as ``_LinearSwiGLUFn`` and ``_LinearFn``; keeps the same tensors.  Backward: the gradient of the activation never
+    leaves the down projection's dgrad kernel, whose epilogue turns it into ``d(gate) | d(up)``."""
+
+    @staticmethod
+    def forward(ctx, x2, w, bias, wd, res2):
+        gu, act = _linear_swiglu_forward(x2, w, bias)
+        y = gemm(act, wd, addend=res2)
+        ctx.save_for_backward(x2, w, gu, act, wd)
+        ctx.has_bias, ctx.has_res = bias is not None, res2 is not None
+        ctx.weight_refs = tuple(weakref.ref(t) if hasattr(t, "_cb_grad_out") else None for t in (w, wd))
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x2, w, gu, act, wd = ctx.saved_tensors
+        dy2 = dy.reshape(-1, dy.shape[-1])
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
+        need_x, need_w, need_b, need_wd, need_res = ctx.needs_input_grad
+        need_b = need_b and ctx.has_bias
+        dest = [grad_destination(r()) if r is not None and need else None for r, need in zip(ctx.weight_refs, (need_w, need_wd))]
+        dx = dw = db = dwd = None
+        if need_x or need_w or need_b:
+            M, I2 = gu.shape
+            dgu = torch.empty_like(gu)
+            code = _ext.lib().cb_gemm2sm_bf16_glu_bwd(
+                dy2.data_ptr(), wd.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, I2 // 2, dy2.shape[1], dy2.stride(0), wd.stride(0),
+                gu.stride(0), dgu.stride(0), _ext.status_buffer(dy2.device).data_ptr(), _ext.stream_ptr())
+            if code > 0:
+                _ext.check(code, "gemm2sm_bf16_glu_bwd")
+            if code != 0:                                        # shape not covered: dgrad, then the activation's backward
+                dgu = _glu_backward(gemm(dy2, wd, b_mn=True), gu)
+            if need_x:
+                dx = gemm(dgu, w, b_mn=True)
+        if need_wd:
+            dwd = wgrad(dy2, act, out=dest[1])
+        if need_w:
+            dw = wgrad(dgu, x2, out=dest[0])
+        if need_b:
+            db = colsum(dgu)
+        return dx, dw, db, dwd, dy2 if ctx.has_res and need_res else None
+
+
+def swiglu_mlp(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, bias: Optional[torch.Tensor] = None,
+               residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``linear(linear_swiglu(x, w_gate_up, bias), w_down, residual=residual)``: the gated MLP of a decoder layer as one
+    autograd node, for the cases that :func:`linear_swiglu` fuses."""
+    if (_FUSED_GLU != "0" and _fast(x, w_gate_up, w_down, bias, residual) and w_gate_up.shape[0] % 256 == 0 and x.shape[-1] % 8 == 0
+            and w_down.shape[0] % 8 == 0 and w_gate_up.stride(1) == 1 and w_down.is_contiguous()
+            and _ext.has_symbol("cb_gemm2sm_bf16_glu_bwd")):
+        x2 = x.reshape(-1, x.shape[-1])
+        if not x2.is_contiguous():
+            x2 = x2.contiguous()
+        res2 = residual.reshape(-1, w_down.shape[0]) if residual is not None else None
+        y = _SwiGLUMLPFn.apply(x2, w_gate_up, bias, w_down, res2)
+        return y if x.dim() == 2 else y.view(*x.shape[:-1], w_down.shape[0])
+    return linear(linear_swiglu(x, w_gate_up, bias), w_down, residual=residual)
 
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:

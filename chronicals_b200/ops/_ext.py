@@ -57,6 +57,7 @@ _PROTOTYPES = {
     "cb_gemm2sm_bf16_ex": [P, P, P, P, P, I, I, I, L, L, L, L, I, I, I, I, I, P, P],
     "cb_gemm2sm_cost_ns": [I, I, I, I, I, I],
     "cb_gemm2sm_bf16_dual": [P, P, P, P, P, P, P, I, I, I, I, L, L, L, L, L, L, I, P, P],
+    "cb_gemm2sm_bf16_glu_bwd": [P, P, P, P, I, I, I, L, L, L, L, P, P],
     "cb_gemm2sm_bf16_glu": [P, P, P, P, P, I, I, I, L, L, L, L, P, P],
     "cb_lora_pack": [P, P, P, P, P, P, I, I, I, P, P, P],
     "cb_lora_unpack": [P, P, P, P, I, I, I, P, P, P, P],

@@ -28,3 +28,30 @@ def test_chosen_kernel(M, N, K, a_mn, b_mn, fp32):
     # fp32 sums of K products of order one, one rounding of the result
     slack = K ** 0.5 * 2e-6 * 8 + (0 if fp32 else 1e-6)
     assert ((out.double() - want).abs() <= (1e-6 if fp32 else 2.0 ** -8) * want.abs() + slack * 4).all()
+
+
+# one row, ragged row tiles, a last tile of 128 activation columns, frozen weights; with and without bias and residual
+@pytest.mark.parametrize("T,H,I", [(1, 64, 128), (300, 896, 640), (513, 256, 1408), (130, 72, 256)])
+@pytest.mark.parametrize("extras,frozen", [(False, False), (True, False), (True, True)])
+def test_swiglu_mlp_gradients(T, H, I, extras, frozen):
+    g = torch.Generator(device=DEV).manual_seed(T + I)
+
+    def r(*shape, scale=1.0):
+        return (scale * torch.randn(*shape, device=DEV, generator=g)).to(torch.bfloat16)
+    x, wg, wd, dy = r(T, H), r(2 * I, H, scale=H ** -0.5), r(H, I, scale=I ** -0.5), r(T, H)
+    b, res = (r(2 * I, scale=0.1), r(T, H)) if extras else (None, None)
+    leaves = [t for t in (x, b, res) if t is not None] + ([] if frozen else [wg, wd])
+    for t in leaves:
+        t.requires_grad_()
+    y = ops.swiglu_mlp(x, wg, wd, b, res)
+    y.backward(dy)
+    _ext.check_status()
+    got = [y] + [t.grad for t in leaves]
+    up = {id(t): t.detach().double().requires_grad_() for t in (x, wg, wd, b, res) if t is not None}
+    gate, lin = (up[id(x)] @ up[id(wg)].t() + (up[id(b)] if extras else 0)).chunk(2, dim=1)
+    want = (torch.nn.functional.silu(gate) * lin) @ up[id(wd)].t() + (up[id(res)] if extras else 0)
+    want.backward(dy.double())
+    for a, w in zip(got, [want] + [up[id(t)].grad for t in leaves]):
+        # gate | up, the activation (by tanh.approx, 2^-11) and d(gate) | d(up) are rounded to bf16 on the way
+        assert ((a.double() - w).norm() <= 2.0 ** -7 * w.norm() + 1e-6).item()
+    assert frozen is False or (wg.grad is None and wd.grad is None)

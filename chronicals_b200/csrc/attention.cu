@@ -2016,7 +2016,7 @@ int cb_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
 }
 
 #ifdef CB_ATTN_PHASE_TIMERS
-// out[2][16] cycles per phase (see CB_PHASE in attn_bwd2_kernel), slot 15 = number of CTAs; clears the table
+// out[2][16] cycles per phase (see CB_PHASE in the kernels), slot 15 = number of CTAs; clears the table
 int cb_attn_phase_read(unsigned long long* out) {
   CB_CHECK_CUDA(cudaDeviceSynchronize());
   CB_CHECK_CUDA(cudaMemcpyFromSymbol(out, cb::cb_attn_phase, sizeof(unsigned long long) * 32));

@@ -145,3 +145,27 @@ def test_linear_cross_entropy_splits(T, V, smoothing):
     rows = ops.linear_cross_entropy(h, w, y, label_smoothing=smoothing, reduction="none")
     want = torch.nn.functional.cross_entropy(h.double() @ w.double().t(), y, label_smoothing=smoothing, reduction="none")
     assert (rows.double() - want).abs().max().item() < 2e-5 * max(1.0, want.abs().max().item())      # fp32 sums throughout
+
+
+# less than a load, less than and just past the four loads in flight, a chunk and one value more, a base off the 16-byte boundary
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("master", [False, True])
+def test_adamw_norm_and_update_at_the_edges_of_a_chunk(dtype, master):
+    from chronicals_b200.optimizers.fused_adamw import FusedAdamW
+    g = _gen(3)
+    sizes = [1, 3, 7, 2048, 4095, 6151, 8191, 8192, 8193, 20000, 9 * 8192 + 5]
+    params = [torch.nn.Parameter(torch.randn(n, device=DEV, generator=g).to(dtype)) for n in sizes]
+    for i, p in enumerate(params):
+        grad = torch.randn(sizes[i] + 1, device=DEV, generator=g).to(dtype)
+        p.grad = grad[1:] if i % 2 else grad[:-1]
+    opt = FusedAdamW(params, lr=1e-2, weight_decay=0.1, max_grad_norm=1.0, master_weights=master)
+    before = [p.detach().double() for p in params]
+    opt.step()
+    norm = sum(p.grad.double().square().sum() for p in params).sqrt()
+    assert abs(opt.last_grad_norm.double() - norm).item() < 1e-5 * norm.item()       # fp32 sums of 8192 squares, fp64 beyond
+    clip = 1.0 / (norm + 1e-6)
+    for p, b in zip(params, before):
+        gr = p.grad.double() * clip
+        want = b * (1 - 1e-3) - 1e-2 * gr / (gr.abs() + 1e-8)                        # first step: m / bc1 = g, v / bc2 = g^2
+        eps = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6
+        assert ((p.detach().double() - want).abs() <= eps * want.abs() + 2e-6).all()

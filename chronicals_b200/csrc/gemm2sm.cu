@@ -808,7 +808,9 @@ PairPlan plan_pairs(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool
     if (best.bn == 0 || whole * (1.0 + 0.12 * std::min(1.0, whole / 150.0)) < best.us) best = {bn, false, whole};
     // pairs at different depths of K share no operands, which a very long K does not forgive unless most tiles are whole
     // (2624 x 3584 x 37,888: 681 us against 512); below 32 k-blocks the fixups of many small runs outweigh the estimate
-    if (may_split && T % pairs != 0 && kb >= 32 && (kb <= 256 || T >= 3 * pairs)) {
+    // and the last round has to be empty by more than the fixups, 72 k-blocks' time, take
+    if (may_split && T % pairs != 0 && kb >= 32 && (kb <= 256 || T >= 3 * pairs) &&
+        static_cast<double>(T) / pairs + 72.0 / kb < (T + pairs - 1) / pairs - 0.05) {
       const double split = split_fixed[i] + split_kb[i] * kb * T / pairs;
       if (split < 1.05 * best.us) best = {bn, true, split};     // 1.05: whole tiles are the ones estimated too low here
     }

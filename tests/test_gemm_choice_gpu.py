@@ -12,7 +12,9 @@ DEV = "cuda"
 # 128-wide single-CTA tiles, 256-wide ones, pairs of 256, 224 and 192, tiles cut along K; ragged last tiles in M and N, K that
 # is no multiple of the k-block
 @pytest.mark.parametrize("M,N,K", [(1000, 896, 1152), (512, 1152, 896), (128, 896, 4864), (2624, 2048, 1096), (4096, 1536, 1000),
-                                   (3000, 1800, 520), (1500, 3584, 1024), (1008, 200, 2056), (9728, 896, 4104), (304, 5120, 328)])
+                                   (3000, 1800, 520), (1500, 3584, 1024), (1008, 200, 2056), (9728, 896, 4104), (304, 5120, 328),
+                                   # outputs as narrow as an adapter's rank
+                                   (8192, 32, 2056), (300, 48, 896), (1000, 64, 520), (256, 16, 4104), (136, 8, 72)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
 @pytest.mark.parametrize("fp32", [False, True])
 def test_chosen_kernel(M, N, K, a_mn, b_mn, fp32):

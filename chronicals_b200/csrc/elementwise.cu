@@ -9,6 +9,7 @@
 // patches in.
 #include <algorithm>
 #include <cstring>
+#include <utility>
 #include <cooperative_groups.h>
 #include "common.cuh"
 
@@ -696,6 +697,11 @@ ce_logits_kernel(const T* __restrict__ logits, const long long* __restrict__ lab
     }
     return;
   }
+  // the first block's shared memory may be written only once that block is known to run: everybody arrives here, and whoever
+  // writes waits before it does, a row's reading later
+  cg::cluster_group cl = cg::this_cluster();
+  cg::cluster_group::arrival_token started;
+  if (gridDim.y > 1) started = cl.barrier_arrive();
   const T* lp = logits + row * ld;
   const int head = ce_head(lp, V), nvec = (V - head) / N, tail0 = head + nvec * N;
   const uint4* vp = reinterpret_cast<const uint4*>(lp + head);
@@ -748,7 +754,7 @@ ce_logits_kernel(const T* __restrict__ logits, const long long* __restrict__ lab
     for (int i = 0; i < EW_THREADS / 32; ++i) a.merge(sm[i], ss[i], sl[i]);
   }
   if (gridDim.y > 1) {
-    cg::cluster_group cl = cg::this_cluster();
+    cl.barrier_wait(std::move(started));
     if (threadIdx.x == 0) {
       float* dst = cl.map_shared_rank(&part[0][0], 0);
       dst[blockIdx.y] = a.m;

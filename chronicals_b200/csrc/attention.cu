@@ -1506,136 +1506,135 @@ attn_bwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     return ok;
   };
 
-  if (warp >= 14) {
-    reg_dec<BWD3_REGS_ISSUE>();
-  } else if (warp == 13) {
-    reg_dec<BWD3_REGS_ISSUE>();
-    // ------------------------------------------------------------------ loads
-    const int u_start = __shfl_sync(0xffffffffu, start, 0);
-    const int u_jb = __shfl_sync(0xffffffffu, jb, 0);
-    const int u_n = __shfl_sync(0xffffffffu, n_it, 0);
-    float lse_n[4], dlt_n[4];                          // statistics of the next block: the loads fly an iteration ahead
-    auto fetch_stats = [&](int it) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int rg = (u_jb + it) * 128 + lane + 32 * k;
-        const long long at = static_cast<long long>(h) * a.T + u_start + rg;
-        const bool in = it < u_n && rg < len;
-        lse_n[k] = in ? __ldg(a.lse + at) : 0.f;
-        dlt_n[k] = in ? __ldg(a.delta + at) : 0.f;
-      }
-    };
-    fetch_stats(0);
-    if (elect_one()) {
-      mbar_expect_tx(k_full, L::TILE);                 // K and Q first: S(0) needs no more
-#pragma unroll
-      for (int p = 0; p < PANELS; ++p) tma_load_2d(sK + p * 16384, &tmK, k_full, hkv * D + p * 64, u_start + u_jb * 128);
-    }
-    for (int it = 0; it < u_n; ++it) {
-      const int st = it & 1;
-      const int row0 = u_start + (u_jb + it) * 128;
-      if (it >= 2 && !wait_w(q_empty + st, (it >> 1) - 1, CB_ERR_WAIT_EMPTY)) break;
+  if (warp >= 12) {
+    reg_dec<BWD3_REGS_ISSUE>();        // the whole warpgroup at one place, before its warps part
+    if (warp == 13) {
+      // ------------------------------------------------------------------ loads
+      const int u_start = __shfl_sync(0xffffffffu, start, 0);
+      const int u_jb = __shfl_sync(0xffffffffu, jb, 0);
+      const int u_n = __shfl_sync(0xffffffffu, n_it, 0);
+      float lse_n[4], dlt_n[4];                          // statistics of the next block: the loads fly an iteration ahead
+      auto fetch_stats = [&](int it) {
+  #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int rg = (u_jb + it) * 128 + lane + 32 * k;
+          const long long at = static_cast<long long>(h) * a.T + u_start + rg;
+          const bool in = it < u_n && rg < len;
+          lse_n[k] = in ? __ldg(a.lse + at) : 0.f;
+          dlt_n[k] = in ? __ldg(a.delta + at) : 0.f;
+        }
+      };
+      fetch_stats(0);
       if (elect_one()) {
-        mbar_expect_tx(q_full + st, L::TILE);
-#pragma unroll
-        for (int p = 0; p < PANELS; ++p) tma_load_2d(sQ + st * L::TILE + p * 16384, &tmQ, q_full + st, h * D + p * 64, row0);
-        if (it == 0) {
-          mbar_expect_tx(v_full, L::TILE);
-#pragma unroll
-          for (int p = 0; p < PANELS; ++p) tma_load_2d(sV + p * 16384, &tmV, v_full, hkv * D + p * 64, row0);
+        mbar_expect_tx(k_full, L::TILE);                 // K and Q first: S(0) needs no more
+  #pragma unroll
+        for (int p = 0; p < PANELS; ++p) tma_load_2d(sK + p * 16384, &tmK, k_full, hkv * D + p * 64, u_start + u_jb * 128);
+      }
+      for (int it = 0; it < u_n; ++it) {
+        const int st = it & 1;
+        const int row0 = u_start + (u_jb + it) * 128;
+        if (it >= 2 && !wait_w(q_empty + st, (it >> 1) - 1, CB_ERR_WAIT_EMPTY)) break;
+        if (elect_one()) {
+          mbar_expect_tx(q_full + st, L::TILE);
+  #pragma unroll
+          for (int p = 0; p < PANELS; ++p) tma_load_2d(sQ + st * L::TILE + p * 16384, &tmQ, q_full + st, h * D + p * 64, row0);
+          if (it == 0) {
+            mbar_expect_tx(v_full, L::TILE);
+  #pragma unroll
+            for (int p = 0; p < PANELS; ++p) tma_load_2d(sV + p * 16384, &tmV, v_full, hkv * D + p * 64, row0);
+          }
+        }
+        // rows past the end of the document get lse = +inf: their probabilities are exact zeros
+  #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const bool in = (u_jb + it) * 128 + lane + 32 * k < len;
+          sStat[st * 256 + lane + 32 * k] = in ? lse_n[k] * LOG2E : INFINITY;
+          sStat[st * 256 + 128 + lane + 32 * k] = dlt_n[k];
+        }
+        arrive_w(st_full + st);
+        fetch_stats(it + 1);
+        const int sd = it % NDO;
+        if (it >= NDO && !wait_w(do_empty + sd, it / NDO - 1, CB_ERR_WAIT_EMPTY)) break;
+        if (elect_one()) {
+          mbar_expect_tx(do_full + sd, L::TILE);
+  #pragma unroll
+          for (int p = 0; p < PANELS; ++p) tma_load_2d(sdO + sd * L::TILE + p * 16384, &tmdO, do_full + sd, h * D + p * 64, row0);
         }
       }
-      // rows past the end of the document get lse = +inf: their probabilities are exact zeros
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const bool in = (u_jb + it) * 128 + lane + 32 * k < len;
-        sStat[st * 256 + lane + 32 * k] = in ? lse_n[k] * LOG2E : INFINITY;
-        sStat[st * 256 + 128 + lane + 32 * k] = dlt_n[k];
+      __syncwarp();
+    } else if (warp == 12) {
+      // ------------------------------------------------------------------ MMA issue
+      const int u_n = __shfl_sync(0xffffffffu, n_it, 0);
+      const uint32_t u_tmem = __shfl_sync(0xffffffffu, tmem, 0);
+      const uint32_t kA = smem_u32(sK), vA = smem_u32(sV), dsA = smem_u32(sdS);
+      auto issue_s = [&](int it) {                       // S^T(it) = K Q(it)^T
+        if (!wait_w(q_full + (it & 1), it >> 1, CB_ERR_WAIT_FULL)) return;
+        const uint32_t qA = smem_u32(sQ + (it & 1) * L::TILE);
+        tc_fence_after();
+        if (elect_one()) {
+  #pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            umma_f16_ss(u_tmem + C_S, desc_kmajor(kA, kk), desc_kmajor(qA, kk), IDESC_S, kk != 0);
+          umma_commit(s_full);
+        }
+      };
+      auto issue_dp = [&](int it) {                      // dP^T(it) = V dO(it)^T
+        if (!wait_w(do_full + it % NDO, it / NDO, CB_ERR_WAIT_FULL)) return;
+        const uint32_t doA = smem_u32(sdO + (it % NDO) * L::TILE);
+        tc_fence_after();
+        if (elect_one()) {
+  #pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            umma_f16_ss(u_tmem + C_DP, desc_kmajor(vA, kk), desc_kmajor(doA, kk), IDESC_S, kk != 0);
+          umma_commit(dp_full);
+        }
+      };
+      wait_w(k_full, 0, CB_ERR_WAIT_FULL);
+      if (ok) issue_s(0);
+      if (ok && wait_w(v_full, 0, CB_ERR_WAIT_FULL)) issue_dp(0);
+      CB_PHASE(12);
+      for (int it = 0; it < u_n && ok; ++it) {
+        if (!wait_w(p_ready, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
+        CB_PHASE(0);
+        const uint32_t doA = smem_u32(sdO + (it % NDO) * L::TILE);
+        tc_fence_after();
+        if (elect_one()) {
+  #pragma unroll
+          for (int kk = 0; kk < 8; ++kk)                 // dV += P^T dO, A from TMEM: 16 queries = 8 words a step
+            umma_f16_ts(u_tmem + C_DV, u_tmem + C_S + (kk >> 1) * 32 + (kk & 1) * 8, desc_mnmajor(doA, kk), IDESC_KV, (it | kk) != 0);
+          umma_commit(do_empty + it % NDO);
+        }
+        if (it + 1 < u_n) issue_s(it + 1);               // over S(it), P(it): both are consumed, MMAs complete in order
+        CB_PHASE(1);
+        if (!ok || !wait_w(ds_ready, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
+        CB_PHASE(2);
+        if (DQ_APART) {                                  // dP(it + 1) needs nothing of this dQ: first, so that dS is not kept waiting
+          if (it + 1 < u_n) issue_dp(it + 1);
+          if (!ok || (it > 0 && !wait_w(dq_free, it - 1, CB_ERR_WAIT_TMEM_EMPTY))) break;
+        }
+        const uint32_t qA = smem_u32(sQ + (it & 1) * L::TILE);
+        tc_fence_after();
+        if (elect_one()) {
+  #pragma unroll
+          for (int kk = 0; kk < 8; ++kk)                 // dQ = dS K (D = 128: over the columns of dP)
+            umma_f16_ss(u_tmem + C_DQ, desc_mnmajor(dsA, kk), desc_mnmajor(kA, kk), IDESC_DQ, kk != 0);
+          umma_commit(dq_full);
+  #pragma unroll
+          for (int kk = 0; kk < 8; ++kk)                 // dK += dS^T Q
+            umma_f16_ss(u_tmem + C_DK, desc_kmajor(dsA, kk), desc_mnmajor(qA, kk), IDESC_KV, (it | kk) != 0);
+          umma_commit(ds_free);
+          umma_commit(q_empty + (it & 1));
+        }
+        CB_PHASE(3);
+        if (!DQ_APART && it + 1 < u_n) {
+          if (!wait_w(dq_free, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
+          CB_PHASE(4);
+          issue_dp(it + 1);
+          CB_PHASE(5);
+        }
       }
-      arrive_w(st_full + st);
-      fetch_stats(it + 1);
-      const int sd = it % NDO;
-      if (it >= NDO && !wait_w(do_empty + sd, it / NDO - 1, CB_ERR_WAIT_EMPTY)) break;
-      if (elect_one()) {
-        mbar_expect_tx(do_full + sd, L::TILE);
-#pragma unroll
-        for (int p = 0; p < PANELS; ++p) tma_load_2d(sdO + sd * L::TILE + p * 16384, &tmdO, do_full + sd, h * D + p * 64, row0);
-      }
+      __syncwarp();
     }
-    __syncwarp();
-  } else if (warp == 12) {
-    reg_dec<BWD3_REGS_ISSUE>();
-    // ------------------------------------------------------------------ MMA issue
-    const int u_n = __shfl_sync(0xffffffffu, n_it, 0);
-    const uint32_t u_tmem = __shfl_sync(0xffffffffu, tmem, 0);
-    const uint32_t kA = smem_u32(sK), vA = smem_u32(sV), dsA = smem_u32(sdS);
-    auto issue_s = [&](int it) {                       // S^T(it) = K Q(it)^T
-      if (!wait_w(q_full + (it & 1), it >> 1, CB_ERR_WAIT_FULL)) return;
-      const uint32_t qA = smem_u32(sQ + (it & 1) * L::TILE);
-      tc_fence_after();
-      if (elect_one()) {
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16_ss(u_tmem + C_S, desc_kmajor(kA, kk), desc_kmajor(qA, kk), IDESC_S, kk != 0);
-        umma_commit(s_full);
-      }
-    };
-    auto issue_dp = [&](int it) {                      // dP^T(it) = V dO(it)^T
-      if (!wait_w(do_full + it % NDO, it / NDO, CB_ERR_WAIT_FULL)) return;
-      const uint32_t doA = smem_u32(sdO + (it % NDO) * L::TILE);
-      tc_fence_after();
-      if (elect_one()) {
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16_ss(u_tmem + C_DP, desc_kmajor(vA, kk), desc_kmajor(doA, kk), IDESC_S, kk != 0);
-        umma_commit(dp_full);
-      }
-    };
-    wait_w(k_full, 0, CB_ERR_WAIT_FULL);
-    if (ok) issue_s(0);
-    if (ok && wait_w(v_full, 0, CB_ERR_WAIT_FULL)) issue_dp(0);
-    CB_PHASE(12);
-    for (int it = 0; it < u_n && ok; ++it) {
-      if (!wait_w(p_ready, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
-      CB_PHASE(0);
-      const uint32_t doA = smem_u32(sdO + (it % NDO) * L::TILE);
-      tc_fence_after();
-      if (elect_one()) {
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)                 // dV += P^T dO, A from TMEM: 16 queries = 8 words a step
-          umma_f16_ts(u_tmem + C_DV, u_tmem + C_S + (kk >> 1) * 32 + (kk & 1) * 8, desc_mnmajor(doA, kk), IDESC_KV, (it | kk) != 0);
-        umma_commit(do_empty + it % NDO);
-      }
-      if (it + 1 < u_n) issue_s(it + 1);               // over S(it), P(it): both are consumed, MMAs complete in order
-      CB_PHASE(1);
-      if (!ok || !wait_w(ds_ready, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
-      CB_PHASE(2);
-      if (DQ_APART) {                                  // dP(it + 1) needs nothing of this dQ: first, so that dS is not kept waiting
-        if (it + 1 < u_n) issue_dp(it + 1);
-        if (!ok || (it > 0 && !wait_w(dq_free, it - 1, CB_ERR_WAIT_TMEM_EMPTY))) break;
-      }
-      const uint32_t qA = smem_u32(sQ + (it & 1) * L::TILE);
-      tc_fence_after();
-      if (elect_one()) {
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)                 // dQ = dS K (D = 128: over the columns of dP)
-          umma_f16_ss(u_tmem + C_DQ, desc_mnmajor(dsA, kk), desc_mnmajor(kA, kk), IDESC_DQ, kk != 0);
-        umma_commit(dq_full);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)                 // dK += dS^T Q
-          umma_f16_ss(u_tmem + C_DK, desc_kmajor(dsA, kk), desc_mnmajor(qA, kk), IDESC_KV, (it | kk) != 0);
-        umma_commit(ds_free);
-        umma_commit(q_empty + (it & 1));
-      }
-      CB_PHASE(3);
-      if (!DQ_APART && it + 1 < u_n) {
-        if (!wait_w(dq_free, it, CB_ERR_WAIT_TMEM_EMPTY)) break;
-        CB_PHASE(4);
-        issue_dp(it + 1);
-        CB_PHASE(5);
-      }
-    }
-    __syncwarp();
   } else if (warp >= 8) {
     reg_inc<BWD3_REGS_DQ>();
     // ------------------------------------------------------------------ dQ: TMEM -> shared memory -> TMA reduce-add

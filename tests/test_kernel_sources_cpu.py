@@ -50,3 +50,19 @@ def test_a_cluster_meets_before_one_block_touches_the_memory_of_another():
         split = re.search(r"barrier_arrive\(\).*barrier_wait\(", before, re.S)
         assert whole or split, f"{path}: {name}"
     assert seen >= 2
+
+
+def test_a_warpgroup_changes_its_registers_at_one_place():
+    """``setmaxnreg`` is one instruction for all four warps of a warpgroup: no branch inside a warpgroup may lie before it."""
+    seen = 0
+    for path, name, body in _kernels():
+        changes = list(re.finditer(r"reg_(?:inc|dec)<(\w+)>\(\)", body))
+        for m in changes:
+            seen += 1
+            assert sum(c.group(0) == m.group(0) for c in changes) == 1, f"{path}: {name}: {m.group(0)} in more than one branch"
+            opened = [c for c in re.finditer(r"if \(warp (\S+) (\w+)\) \{", body[:m.start()])
+                      if _closing(body, c.end() - 1) > m.start()]     # the conditions that hold where it stands
+            for c in opened:
+                bound = int(c.group(2))
+                assert c.group(1) in (">=", "<") and bound % 4 == 0, f"{path}: {name}: {c.group(0)}"
+    assert seen >= 3

@@ -171,8 +171,14 @@ class Attention(nn.Module):
         return self.o_proj(o, residual)
 
 
-def _has_hooks(m: nn.Module) -> bool:
-    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+def _is_one_product(m: nn.Module) -> bool:
+    """Calling ``m`` is one product with ``m.weight`` and nothing else: no other class or patched ``forward``, no adapter, FP8 path
+    or bias, and no hook, its own or one registered for all modules, that waits for the call."""
+    hooks = torch.nn.modules.module
+    return (type(m) is FusedLinear and "forward" not in m.__dict__ and m.is_plain() and m.bias is None
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                     or hooks._global_forward_hooks or hooks._global_forward_pre_hooks
+                     or hooks._global_backward_hooks or hooks._global_backward_pre_hooks))
 
 
 class MLP(nn.Module):
@@ -187,7 +193,7 @@ class MLP(nn.Module):
     def forward(self, x, residual):
         fl, down = self.gate_up_proj, self.down_proj
         if not self.gelu and fl.is_plain():
-            if down.is_plain() and down.bias is None and not _has_hooks(down):
+            if _is_one_product(down):
                 return ops.swiglu_mlp(x, fl.weight, down.weight, fl.bias, residual)       # the whole block as one autograd node
             a = ops.linear_swiglu(x, fl.weight, fl.bias)       # activation in the projection's epilogue
         else:

@@ -192,8 +192,12 @@ def check(code: int, what: str) -> None:
 
 def stream_ptr() -> int:
     """Handle of the calling thread's current stream on its current device.  Asked of the runtime on every launch;
-    ``torch.cuda.current_stream()`` builds a stream object for the same answer (6 us of a launch's 34)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    ``torch.cuda.current_stream()`` builds a stream object for the same answer (6 us of a launch's 34); it is asked where
+    torch does not have the two functions, which are not part of its documented interface."""
+    try:
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    except AttributeError:
+        return torch.cuda.current_stream().cuda_stream
 
 
 def status_buffer(device: Optional[torch.device] = None) -> torch.Tensor:

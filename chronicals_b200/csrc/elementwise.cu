@@ -8,6 +8,7 @@
 // :1448-1625 QK-RoPE, :127-210 cross-entropy) and the Liger kernels its trainer
 // patches in.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <utility>
 #include <cooperative_groups.h>
@@ -933,11 +934,24 @@ RowPlan row_plan(int N) {
   return {0, 0, 0};
 }
 constexpr int RMS_BWD_RING2 = 3, RMS_BWD_RING4 = 2;   // ring depth by vectors a thread
+constexpr int RMS_MAX_DEVICES = 64;
 
+// Dynamic shared memory that a backward kernel may be launched with on the current device.  A kernel's limit is one for all host
+// threads, so it is raised once, to what the widest row of either layout takes with all three inputs, and never lowered again:
+// set to a call's own size, it could shrink between another thread's setting and its launch, which then failed.
+constexpr int RMS_BWD_SMEM_MAX = 96 * 1024;
+static_assert(RMS_BWD_RING2 * 3 * 2 * 320 * 16 <= RMS_BWD_SMEM_MAX && RMS_BWD_RING4 * 3 * 4 * cb::EW_THREADS * 16 <= RMS_BWD_SMEM_MAX,
+              "ring of the widest row");
 template <typename K>
-int rms_smem(K kern, size_t bytes) {
-  if (bytes <= 40 * 1024) return 0;                    // with the kernels' static arrays within the default 48 KB
-  return static_cast<int>(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+int allow_rms_smem(K kern, std::atomic<bool>* raised_on_device) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const bool known = dev < RMS_MAX_DEVICES;
+  if (known && raised_on_device[dev].load(std::memory_order_acquire)) return 0;
+  const int r = static_cast<int>(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RMS_BWD_SMEM_MAX));
+  if (r == 0 && known) raised_on_device[dev].store(true, std::memory_order_release);
+  return r;
 }
 
 int launch_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const void* dres_in, void* dx,
@@ -946,17 +960,18 @@ int launch_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float
   const int ring = pl.vpl == 2 ? RMS_BWD_RING2 : RMS_BWD_RING4;
   size_t smem = static_cast<size_t>(ring) * (dres_in ? 3 : 2) * pl.vpl * pl.threads * 16;
   if (pl.rows > 1) smem = std::max(smem, static_cast<size_t>(pl.rows) * N * sizeof(float));
-  const auto go = [&](auto kern) {
-    const int e = rms_smem(kern, smem);
+  static std::atomic<bool> raised[3][RMS_MAX_DEVICES] = {};
+  const auto go = [&](auto kern, std::atomic<bool>* raised_on_device) {
+    const int e = allow_rms_smem(kern, raised_on_device);
     if (e) return e;
     kern<<<grid, pl.threads, smem, s>>>(static_cast<const cb::bf16*>(dy), static_cast<const cb::bf16*>(h),
                                         static_cast<const cb::bf16*>(w), rstd, static_cast<const cb::bf16*>(dres_in),
                                         static_cast<cb::bf16*>(dx), part, M, N, offset);
     return static_cast<int>(cudaGetLastError());
   };
-  if (pl.rows > 1) return go(cb::rmsnorm_bwd_kernel<4, true, RMS_BWD_RING4>);
-  if (pl.vpl == 2) return go(cb::rmsnorm_bwd_kernel<2, false, RMS_BWD_RING2>);
-  return go(cb::rmsnorm_bwd_kernel<4, false, RMS_BWD_RING4>);
+  if (pl.rows > 1) return go(cb::rmsnorm_bwd_kernel<4, true, RMS_BWD_RING4>, raised[0]);
+  if (pl.vpl == 2) return go(cb::rmsnorm_bwd_kernel<2, false, RMS_BWD_RING2>, raised[1]);
+  return go(cb::rmsnorm_bwd_kernel<4, false, RMS_BWD_RING4>, raised[2]);
 }
 }  // namespace
 

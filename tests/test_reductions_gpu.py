@@ -1,5 +1,6 @@
 """Reductions over rows, runs and columns at the sizes where their splits can go wrong, against 64-bit formulas."""
 import math
+import threading
 
 import pytest
 import torch
@@ -96,6 +97,36 @@ def test_rmsnorm_layouts(M, N, residual):
     for got, want, slack in ((y, yr, 1e-5), (x.grad, xr.grad, 2e-5), (w.grad, wr.grad, 1e-5 * size + 1e-5)):
         # one rounding to bf16 and fp32 sums (dx of a residual cancels: its terms are of order one)
         assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()
+
+
+def test_rmsnorm_backward_from_two_threads():
+    """Calls that need more and calls that need less shared memory of the same kernel, at the same time."""
+    M, N, calls = 4, 5120, 4000                                   # 90 KB a block with a residual's gradient, 60 KB without
+    L = ops._ext.lib()
+    g = _gen(1)
+    dy, h, res = (torch.randn(M, N, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3))
+    w, rstd = torch.ones(N, device=DEV, dtype=torch.bfloat16), torch.ones(M, device=DEV)
+    failed, ended = [], []
+
+    def run(dres):
+        s = torch.cuda.Stream()
+        dx, dw = torch.empty_like(h), torch.empty_like(w)
+        part = torch.empty(L.cb_rmsnorm_bwd_blocks(M, N) * N, device=DEV)
+        s.wait_stream(torch.cuda.default_stream())
+        for _ in range(calls):
+            code = L.cb_rmsnorm_bwd(dy.data_ptr(), h.data_ptr(), w.data_ptr(), rstd.data_ptr(), dres, dx.data_ptr(), dw.data_ptr(),
+                                    part.data_ptr(), M, N, 0.0, 0, s.cuda_stream)
+            if code != 0:
+                failed.append(code)
+        s.synchronize()
+        ended.append(dres)
+
+    threads = [threading.Thread(target=run, args=(d,)) for d in (res.data_ptr(), None)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed and len(ended) == 2
 
 
 # one block of 32, ragged tiles of 128 in either direction, a pitch, a base off the 16-byte boundary, either copy alone

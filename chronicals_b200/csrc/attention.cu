@@ -1806,15 +1806,15 @@ uint32_t dq[D / 32][32];
 // of 2): a thread takes 8 columns (D is a multiple of 8, so they lie in one section), ATT_FIN_BATCH of them at a time.
 // 8192 tokens, 28 / 4 heads of 128: 32 us (7 TB/s) against 50 with one float4 in flight.
 // clear: write zeros back over every accumulator value read, so that a caller who keeps the scratch buffers between
-// calls never has to clear them again.
+// calls never has to clear them again.  wide: every row of dqkv starts on a 16-byte boundary (else on one of 8 bytes).
 constexpr int ATT_FIN_BATCH = 3;
 __global__ void __launch_bounds__(256)
 attn_bwd_finalize_kernel(float* __restrict__ dq_acc, float* __restrict__ dk_part, float* __restrict__ dv_part,
                          bf16* __restrict__ dqkv, long long ld, int nq, int nk, float scale, const int* __restrict__ cu,
-                         int n_docs, int clear) {
+                         int n_docs, int clear, bool wide) {
   const long long t = blockIdx.x;
   const int total = (nq + 2 * nk) / 8;
-  uint4* out = reinterpret_cast<uint4*>(dqkv + t * ld);
+  bf16* out = dqkv + t * ld;
   const bool valid = t < cu[n_docs];                  // padding tokens get zero gradients
   for (int c0 = threadIdx.x; c0 < total; c0 += ATT_FIN_BATCH * blockDim.x) {
     float4 v[ATT_FIN_BATCH][2];
@@ -1835,8 +1835,14 @@ attn_bwd_finalize_kernel(float* __restrict__ dq_acc, float* __restrict__ dk_part
       const int c = (c0 + i * blockDim.x) * 8;
       if (c < nq + 2 * nk) {
         const float m = c < nq + nk ? scale : 1.f;
-        out[c / 8] = make_uint4(pack_bf16x2(v[i][0].x * m, v[i][0].y * m), pack_bf16x2(v[i][0].z * m, v[i][0].w * m),
-                                pack_bf16x2(v[i][1].x * m, v[i][1].y * m), pack_bf16x2(v[i][1].z * m, v[i][1].w * m));
+        const uint2 lo = make_uint2(pack_bf16x2(v[i][0].x * m, v[i][0].y * m), pack_bf16x2(v[i][0].z * m, v[i][0].w * m));
+        const uint2 hi = make_uint2(pack_bf16x2(v[i][1].x * m, v[i][1].y * m), pack_bf16x2(v[i][1].z * m, v[i][1].w * m));
+        if (wide) {
+          *reinterpret_cast<uint4*>(out + c) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        } else {
+          reinterpret_cast<uint2*>(out + c)[0] = lo;
+          reinterpret_cast<uint2*>(out + c)[1] = hi;
+        }
       }
     }
   }
@@ -1938,7 +1944,8 @@ int cb_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
                 long long ldo, long long ld_do, float scale, float* delta, float* dq_acc, float* dk_part,
                 float* dv_part, void* dqkv, long long ld_dqkv, int* status, void* stream, int scratch_is_zero) {
   if ((D != 64 && D != 128) || hq % hk != 0 || T <= 0 || n_docs <= 0) return -1;
-  if ((reinterpret_cast<uintptr_t>(dqkv) & 15) != 0 || ld_dqkv % 8 != 0) return -1;
+  if ((reinterpret_cast<uintptr_t>(dqkv) & 7) != 0 || ld_dqkv % 4 != 0) return -1;       // the gradient is written 8 bytes at a time
+  const bool wide = (reinterpret_cast<uintptr_t>(dqkv) & 15) == 0 && ld_dqkv % 8 == 0;   // or 16
   CUtensorMap mq, mk, mv, mdo;
   int e = attn_maps(&mq, &mk, &mv, q, k, v, T, hq, hk, D, ldq, ldk, ldv);
   if (e) return e;
@@ -2010,7 +2017,8 @@ int cb_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
   }
   const int vecs = (hq + 2 * hk) * D / 8;
   cb::attn_bwd_finalize_kernel<<<T, std::min(256, (vecs + cb::ATT_FIN_BATCH * 32 - 1) / (cb::ATT_FIN_BATCH * 32) * 32), 0, s>>>(
-      dq_acc, dk_part, dv_part, static_cast<cb::bf16*>(dqkv), ld_dqkv, hq * D, hk * D, scale, cu, n_docs, scratch_is_zero ? 1 : 0);
+      dq_acc, dk_part, dv_part, static_cast<cb::bf16*>(dqkv), ld_dqkv, hq * D, hk * D, scale, cu, n_docs, scratch_is_zero ? 1 : 0,
+      wide);
   return static_cast<int>(cudaGetLastError());
 }
 

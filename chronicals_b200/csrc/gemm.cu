@@ -696,7 +696,7 @@ __global__ void cce_finalize_kernel(const float* __restrict__ loss_rows, const l
 
 // =========================================================================================== host side
 extern "C" int cb_gemm2sm_supported(const void* C, long long ldc, int out_fp32);
-extern "C" int cb_gemm2sm_cost_ns(int M, int N, int K, int a_mn, int b_mn, int out_bytes);
+extern "C" int cb_gemm2sm_cost_ns(int M, int N, int K, int a_mn, int b_mn, int out_bytes, int sms);
 extern "C" int cb_gemm2sm_bf16(const void* A, const void* B, void* C, const void* bias, const void* addend, int M, int N,
                                int K, long long lda, long long ldb, long long ldc, long long ld_add, int a_mn, int b_mn,
                                int out_fp32, int accumulate, int* status, void* stream);
@@ -760,19 +760,22 @@ int pick_block_n(int M, int N, int forced) {
   return best;
 }
 
-// Which kernel: the estimate of the CTA-pair kernel (gemm2sm.cu) against those of the single-CTA kernels, fitted to the same
-// products: rounds of whole tiles over the SMs, a fixed cost that is 2 us lower, and the output.  Returns 0 for pairs, else
-// the single-CTA tile width.  Over those products the choice takes 2.8 % less time on average than the rule by operand size
-// that stood here, 32 % less at most (4096 x 1536 x 8960: 121 -> 83 us) and 6 % more at worst (896 x 4864 x 128: 6.6 -> 7.0).
-int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool pairs_possible) {
+// Which kernel: the estimate of the CTA-pair kernel (gemm2sm.cu) against those of the single-CTA kernels, fitted to 276 products
+// (four model sizes, 128 to 8192 tokens, forward, dgrad and wgrad): rounds of whole tiles over the SMs, a fixed cost that is
+// 2 us lower, and the output.  Returns 0 for pairs, else the single-CTA tile width.  A grid of 128-wide tiles that fits one
+// round is never widened: fewer CTAs would take longer for as many k-blocks (896 x 896 x 128: 5.0 us against 5.9 of 256; the
+// two estimates lie within the fit's error there).  Against the width that pads N least, whatever the rounds: 2.8 % less time
+// on average over those products, 32 % less at most (4096 x 1536 x 8960: 121 -> 83 us).
+int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool pairs_possible, int sms) {
   const bool mn = a_mn && b_mn;
   const double kb = (K + 63) / 64, mb = 1e-6 * M * N * out_bytes;
-  const long long m = (M + 127) / 128, sms = num_sms();
+  const long long m = (M + 127) / 128;
   const long long r128 = (m * ((N + 127) / 128) + sms - 1) / sms, r256 = (m * ((N + 255) / 256) + sms - 1) / sms;
   const double t128 = 4.34 + (mn ? 0.298 : 0.28) * r128 * kb + 0.118 * mb;
   const double t256 = (mn ? 4.43 + 0.35 * r256 : 4.1) + (mn ? 0.382 : 0.358) * r256 * kb + 0.147 * mb;
-  if (pairs_possible && 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes) <= std::min(t128, t256)) return 0;
-  return t128 < t256 ? 128 : 256;
+  const bool narrow = r128 == 1 || t128 < t256;
+  if (pairs_possible && 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes, sms) <= (narrow ? t128 : t256)) return 0;
+  return narrow ? 128 : 256;
 }
 
 // Tensor map of the output for the staged epilogue; returns 0 and sets *ok when C qualifies
@@ -803,6 +806,11 @@ int build_maps(CUtensorMap* ta, CUtensorMap* tb, const void* A, const void* B, i
 
 extern "C" {
 
+// The kernel that cb_gemm_bf16 takes for a product on a chip of `sms` SMs: 0 = CTA pairs, else the single-CTA tile width.
+int cb_gemm_choice(int M, int N, int K, int a_mn, int b_mn, int out_bytes, int sms) {
+  return choose_kernel(M, N, K, a_mn, b_mn, out_bytes, true, sms);
+}
+
 // C[M,N] = A * B^T (+bias) (+addend) (+C).  a_mn / b_mn: 0 when the operand is stored [M|N, K]
 // (K contiguous), 1 when stored [K, M|N].  lda/ldb/ldc/ld_add are row pitches in elements.
 // Returns 0 on a successful launch; negative for rejected arguments; positive CUDA error otherwise.
@@ -814,7 +822,7 @@ int cb_gemm_bf16(const void* A, const void* B, void* C, const void* bias, const 
   // of that width, 2 = CTA-pair kernel
   const bool pairs_possible = cb_gemm2sm_supported(C, ldc, out_fp32) != 0;
   if (force_block_n == 0) {
-    force_block_n = choose_kernel(M, N, K, a_mn, b_mn, out_fp32 ? 4 : 2, pairs_possible);
+    force_block_n = choose_kernel(M, N, K, a_mn, b_mn, out_fp32 ? 4 : 2, pairs_possible, num_sms());
     if (force_block_n == 0) force_block_n = 2;
   }
   if (force_block_n == 2 && pairs_possible)

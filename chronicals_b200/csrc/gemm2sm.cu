@@ -792,7 +792,7 @@ struct PairPlan {
   bool split;
   double us;
 };
-PairPlan plan_pairs(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool may_split, int force_bn) {
+PairPlan plan_pairs(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool may_split, int force_bn, int sms) {
   static const double fixed[3] = {6.0, 6.0, 5.7}, per_mb[3] = {0.112, 0.16, 0.145};       // per MB of output
   static const double per_kb[3] = {0.319, 0.281, 0.265}, per_kb_mn[3] = {0.319, 0.312, 0.309};   // both operands MN-major
   static const double split_fixed[3] = {30.4, 30.6, 26.3}, split_kb[3] = {0.353, 0.33, 0.307};
@@ -801,14 +801,14 @@ PairPlan plan_pairs(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool
   if (!a_mn && N <= 64 && (force_bn == 0 || force_bn == 64)) {
     // an adapter's inner product: wider tiles multiply by zeros for longer than the operand takes to arrive (4096 x 32 x
     // 37,888: 132 us against 149 of 192 columns and 148 of a single CTA's 128; 8192 x 32 x 9728: 42 / 45 / 43)
-    const long long T = (M + 255) / 256, pairs = T < cbhost::num_sms() / 2 ? T : cbhost::num_sms() / 2;
+    const long long T = (M + 255) / 256, pairs = T < sms / 2 ? T : sms / 2;
     best = {64, false, 6.0 + 0.19 * ((T + pairs - 1) / pairs) * kb + per_mb[0] * mb};
   }
   for (int i = 0; i < 3; ++i) {
     const int bn = 256 - 32 * i;
     if (force_bn != 0 && force_bn != bn) continue;
     const long long T = static_cast<long long>((M + 255) / 256) * ((N + bn - 1) / bn);
-    const long long pairs = T < cbhost::num_sms() / 2 ? T : cbhost::num_sms() / 2;
+    const long long pairs = T < sms / 2 ? T : sms / 2;
     const double whole = fixed[i] + (a_mn && b_mn ? per_kb_mn : per_kb)[i] * ((T + pairs - 1) / pairs) * kb + per_mb[i] * mb;
     // a narrower tile reads more per product, which the larger problems feel in L2 and in power
     if (best.bn == 0 || whole * (1.0 + 0.12 * std::min(1.0, whole / 150.0)) < best.us) best = {bn, false, whole};
@@ -880,9 +880,9 @@ int cb_gemm2sm_set_workspace(int device, void* ptr, unsigned long long bytes) {
   return 0;
 }
 
-// What the dispatcher needs to know about a problem: the pair kernel's time in nanoseconds.
-int cb_gemm2sm_cost_ns(int M, int N, int K, int a_mn, int b_mn, int out_bytes) {
-  return static_cast<int>(1e3 * std::min(2e6, plan_pairs(M, N, K, a_mn, b_mn, out_bytes, have_workspace(), 0).us));
+// What the dispatcher needs to know about a problem: the pair kernel's time in nanoseconds on a chip of `sms` SMs.
+int cb_gemm2sm_cost_ns(int M, int N, int K, int a_mn, int b_mn, int out_bytes, int sms) {
+  return static_cast<int>(1e3 * std::min(2e6, plan_pairs(M, N, K, a_mn, b_mn, out_bytes, have_workspace(), 0, sms).us));
 }
 
 // C[M,N] = op(A) * op(B)^T (+bias) (+addend) (+C) on CTA pairs.  Same conventions as cb_gemm_bf16 (gemm.cu):
@@ -896,7 +896,7 @@ int cb_gemm2sm_bf16_ex(const void* A, const void* B, void* C, const void* bias, 
   if (!cb_gemm2sm_supported(C, ldc, out_fp32)) return -2;
   int bn = flags >> 8;
   if (bn != 256 && bn != 224 && bn != 192 && !(bn == 64 && !a_mn && N <= 64)) bn = 0;
-  const PairPlan plan = plan_pairs(M, N, K, a_mn, b_mn, out_fp32 ? 4 : 2, !(flags & 1) && have_workspace(), bn);
+  const PairPlan plan = plan_pairs(M, N, K, a_mn, b_mn, out_fp32 ? 4 : 2, !(flags & 1) && have_workspace(), bn, cbhost::num_sms());
   bn = plan.bn;
   if (b_mn && (ldb * 2) % 16 != 0) return -3;
   CUtensorMap ta, tb, tc, tw;
@@ -1018,7 +1018,7 @@ int cb_gemm2sm_bf16_dual(const void* A, const void* B, const void* A2, const voi
                          long long ldb2, long long ldc, long long ld_add, int b_mn, int* status, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || K2 <= 0) return -1;
   if (!cb_gemm2sm_supported(C, ldc, 0)) return -2;
-  const PairPlan plan = plan_pairs(M, N, K + K2, 0, b_mn, 2, have_workspace(), 0);
+  const PairPlan plan = plan_pairs(M, N, K + K2, 0, b_mn, 2, have_workspace(), 0, cbhost::num_sms());
   const int bn = plan.bn;
   if (b_mn && ((ldb * 2) % 16 != 0 || (ldb2 * 2) % 16 != 0)) return -3;
   CUtensorMap ta, tb, ta2, tb2, tc, tw;

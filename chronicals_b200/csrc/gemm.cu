@@ -766,7 +766,7 @@ int pick_block_n(int M, int N, int forced) {
 // round is never widened: fewer CTAs would take longer for as many k-blocks (896 x 896 x 128: 5.0 us against 5.9 of 256; the
 // two estimates lie within the fit's error there).  Against the width that pads N least, whatever the rounds: 2.8 % less time
 // on average over those products, 32 % less at most (4096 x 1536 x 8960: 121 -> 83 us).
-int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool pairs_possible, int sms) {
+int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool pairs_possible, int sms, double* us = nullptr) {
   const bool mn = a_mn && b_mn;
   const double kb = (K + 63) / 64, mb = 1e-6 * M * N * out_bytes;
   const long long m = (M + 127) / 128;
@@ -774,8 +774,10 @@ int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool p
   const double t128 = 4.34 + (mn ? 0.298 : 0.28) * r128 * kb + 0.118 * mb;
   const double t256 = (mn ? 4.43 + 0.35 * r256 : 4.1) + (mn ? 0.382 : 0.358) * r256 * kb + 0.147 * mb;
   const bool narrow = r128 == 1 || t128 < t256;
-  if (pairs_possible && 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes, sms) <= (narrow ? t128 : t256)) return 0;
-  return narrow ? 128 : 256;
+  const double single = narrow ? t128 : t256;
+  const double pair = pairs_possible ? 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes, sms) : single + 1.0;
+  if (us != nullptr) *us = std::min(single, pair);           // the estimate for the kernel that is taken
+  return pair <= single ? 0 : narrow ? 128 : 256;
 }
 
 // Tensor map of the output for the staged epilogue; returns 0 and sets *ok when C qualifies
@@ -809,6 +811,24 @@ extern "C" {
 // The kernel that cb_gemm_bf16 takes for a product on a chip of `sms` SMs: 0 = CTA pairs, else the single-CTA tile width.
 int cb_gemm_choice(int M, int N, int K, int a_mn, int b_mn, int out_bytes, int sms) {
   return choose_kernel(M, N, K, a_mn, b_mn, out_bytes, true, sms);
+}
+
+// Whether the gated MLP's backward takes the product with the activation's gradient in its epilogue (cb_gemm2sm_bf16_glu_bwd:
+// d(act) [M, I] = dY [M, K] W) or a plain product and the activation's backward kernel, by their estimated times.  The fused
+// kernel runs whole 256-wide tiles on CTA pairs and its epilogue adds to every round, so it wins where d(act)'s way through
+// memory costs more than that: from about 1900 tokens at a width of 896, 700 to 900 at 1536 and 2048, 350 at 3584, 1700 at
+// 5120, and below these where the tiles happen to fill their rounds.
+// Its estimate is fitted to 60 sizes (five model widths, 16 to 16,384 tokens).  Fused / apart, us: K = 896, I = 4864: 64 tokens
+// 15.8 / 11.1, 512 18.0 / 17.4, 1024 25.8 / 25.0, 2048 35.1 / 37.0, 8192 90.5 / 116.2; K = 3584, I = 18,944: 64 36.5 / 30.8,
+// 256 39.7 / 41.6, 1024 109 / 123, 4096 410 / 529.
+int cb_glu_bwd_fused_pays(int M, int I, int K, int sms) {
+  const long long T = static_cast<long long>((M + 255) / 256) * ((I + 255) / 256), pairs = T < sms / 2 ? T : sms / 2;
+  const double kb = (K + 63) / 64;
+  const double fused = 8.3 + ((T + pairs - 1) / pairs) * (3.5 + 0.36 * kb);
+  double dgrad = 0.0;
+  choose_kernel(M, I, K, 0, 1, 2, true, sms, &dgrad);
+  const double apart = dgrad + 2.0 + 1e-6 * M * I * 10 / 6.2;        // three tensors read, two written, 6.2 TB/s
+  return fused <= apart;
 }
 
 // C[M,N] = A * B^T (+bias) (+addend) (+C).  a_mn / b_mn: 0 when the operand is stored [M|N, K]

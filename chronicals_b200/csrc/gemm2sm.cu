@@ -980,7 +980,8 @@ int cb_gemm2sm_bf16_glu(const void* A, const void* W, void* GU, void* ACT, const
 // I a multiple of 64 (returns -5 otherwise).  DACT is neither rounded nor written and read (160 MB at 8192 x 4864); gate and
 // up come by TMA, a chunk ahead of the epilogue, into the room of one of the ring's six stages.
 // Measured at 8192 x 4864, K = 896: 93 us, against 58 for the dgrad and 64 for the activation's backward; it is the epilogue (two
-// special-function and about twenty other instructions a value on four warps) that keeps it from the 58.
+// special-function and about twenty other instructions a value on four warps) that keeps it from the 58.  Always 256-wide whole
+// tiles; which sizes gain by it is cb_glu_bwd_fused_pays's (gemm.cu) to say.
 int cb_gemm2sm_bf16_glu_bwd(const void* DY, const void* WD, const void* GU, void* DGU, int M, int I, int K, long long ld_dy,
                             long long ld_wd, long long ld_gu, long long ld_dgu, int* status, void* stream) {
   if (M <= 0 || I <= 0 || K <= 0) return -1;

@@ -496,11 +496,16 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
     return swiglu(linear(x, w, bias))
 
 
+def _glu_bwd_fused(M: int, I: int, K: int, device: torch.device) -> bool:
+    """The dgrad of the down projection with the activation's backward in its epilogue, rather than one after the other."""
+    return bool(_ext.lib().cb_glu_bwd_fused_pays(M, I, K, _sm_count(device)))
+
+
 class _SwiGLUMLPFn(torch.autograd.Function):
     """``silu(x Wgᵀ + bg) * (x Wuᵀ + bu)`` times the down projection, plus the residual, as one node.
 
-    Forward as ``_LinearSwiGLUFn`` and ``_LinearFn``; keeps the same tensors.  Backward: the gradient of the activation never
-    leaves the down projection's dgrad kernel, whose epilogue turns it into ``d(gate) | d(up)``."""
+    Forward as ``_LinearSwiGLUFn`` and ``_LinearFn``; keeps the same tensors.  Backward: with enough tokens the gradient of the
+    activation never leaves the down projection's dgrad kernel, whose epilogue turns it into ``d(gate) | d(up)``."""
 
     @staticmethod
     def forward(ctx, x2, w, bias, wd, res2):
@@ -523,13 +528,15 @@ class _SwiGLUMLPFn(torch.autograd.Function):
         dx = dw = db = dwd = None
         if need_x or need_w or need_b:
             M, I2 = gu.shape
-            dgu = torch.empty_like(gu)
-            code = _ext.lib().cb_gemm2sm_bf16_glu_bwd(
-                dy2.data_ptr(), wd.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, I2 // 2, dy2.shape[1], dy2.stride(0), wd.stride(0),
-                gu.stride(0), dgu.stride(0), _ext.status_buffer(dy2.device).data_ptr(), _ext.stream_ptr())
-            if code > 0:
-                _ext.check(code, "gemm2sm_bf16_glu_bwd")
-            if code != 0:                                        # shape not covered: dgrad, then the activation's backward
+            code = -1
+            if _glu_bwd_fused(M, I2 // 2, dy2.shape[1], dy2.device):
+                dgu = torch.empty_like(gu)
+                code = _ext.lib().cb_gemm2sm_bf16_glu_bwd(
+                    dy2.data_ptr(), wd.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, I2 // 2, dy2.shape[1], dy2.stride(0),
+                    wd.stride(0), gu.stride(0), dgu.stride(0), _ext.status_buffer(dy2.device).data_ptr(), _ext.stream_ptr())
+                if code > 0:
+                    _ext.check(code, "gemm2sm_bf16_glu_bwd")
+            if code != 0:                                        # few tokens, or not covered: dgrad, then the activation's backward
                 dgu = _glu_backward(gemm(dy2, wd, b_mn=True), gu)
             if need_x:
                 dx = gemm(dgu, w, b_mn=True)

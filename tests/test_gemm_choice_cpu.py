@@ -16,3 +16,14 @@ def test_one_round_of_narrow_tiles_is_not_widened():
             if -(-M // 128) * -(-N // 128) <= 148:
                 assert got != 256, (M, N, K)
     assert seen == {0, 128, 256}
+
+
+# sizes measured on either side of the line (tokens, intermediate size, width); ties left out
+def test_fused_gate_gradient_only_where_it_is_faster():
+    pays = _ext.lib().cb_glu_bwd_fused_pays
+    apart = [(16, 4864, 896), (64, 4864, 896), (256, 4864, 896), (64, 8960, 1536), (256, 8960, 1536), (128, 11008, 2048),
+             (64, 18944, 3584), (128, 18944, 3584), (128, 13824, 5120)]
+    fused = [(2624, 4864, 896), (8192, 4864, 896), (16384, 4864, 896), (1000, 8960, 1536), (8192, 8960, 1536), (1000, 11008, 2048),
+             (8192, 11008, 2048), (512, 18944, 3584), (8192, 18944, 3584), (1000, 13824, 5120), (8192, 13824, 5120)]
+    assert not any(pays(*s, 148) for s in apart)
+    assert all(pays(*s, 148) for s in fused)

@@ -57,3 +57,11 @@ def test_swiglu_mlp_gradients(T, H, I, extras, frozen):
         # gate | up, the activation (by tanh.approx, 2^-11) and d(gate) | d(up) are rounded to bf16 on the way
         assert ((a.double() - w).norm() <= 2.0 ** -7 * w.norm() + 1e-6).item()
     assert frozen is False or (wg.grad is None and wd.grad is None)
+
+
+# both ways of the backward, whichever the sizes would take
+@pytest.mark.parametrize("T,H,I", [(1, 64, 128), (300, 896, 640), (513, 256, 1408), (130, 72, 256)])
+@pytest.mark.parametrize("fused", [True, False])
+def test_swiglu_mlp_gradients_either_way(T, H, I, fused, monkeypatch):
+    monkeypatch.setattr(ops, "_glu_bwd_fused", lambda *a: fused)
+    test_swiglu_mlp_gradients(T, H, I, True, False)

@@ -9,7 +9,6 @@ On a CUDA device the kernel library is mandatory; a missing library raises.
 """
 from __future__ import annotations
 
-import functools
 import math
 import os
 import weakref
@@ -702,29 +701,11 @@ CCE_BWD_CHUNK = 8192               # vocab columns whose d(logits) exist at any 
 CCE_BWD_ELEMENTS = 8192 * 8192     # ... and how many values that is: fewer tokens take wider chunks of the same size
 
 
-@functools.lru_cache(maxsize=256)
 def _cce_chunk(M: int, K: int, V: int, sms: int) -> int:
-    """Vocabulary columns per chunk of the backward: the width (a multiple of the 256-column tile) that costs least, in
-    64-deep k-blocks of one round of tiles.  A chunk is three products, each a whole number of rounds over the SMs, and
-    about 14 k-blocks of launch, fill and drain apiece, so a width is good when it fills its last rounds and chunks are
-    few.  Measured with a 151,936-word vocabulary, K = 896 (forward + backward, chunks of 8192 columns before):
-    64 tokens 1373 -> 858 us, 512 1551 -> 1061, 2048 2666 -> 2341, 4096 4335 -> 4196, 8192 unchanged (chunks of 8192)."""
-    def cdiv(a, b):
-        return -(-a // b)
-    pairs = max(sms // 2, 1)
-    bn = min((256, 224, 192), key=lambda b: cdiv(K, b) * b - K)                # the tile width the products choose
-    nt, width = cdiv(K, bn), bn / 256
-
-    def cost(w):
-        dw = cdiv(cdiv(w, 256) * nt, pairs) * width * cdiv(M, 64)
-        dh = cdiv(cdiv(M, 256) * nt, pairs) * width * cdiv(w, 64)
-        return dw + dh + cdiv(cdiv(M, 128) * cdiv(w, 256), sms) * cdiv(K, 64) + 3 * 14
-    V8 = (V + 7) // 8 * 8
-    top = max(CCE_BWD_CHUNK, CCE_BWD_ELEMENTS // M // 256 * 256)
-    widths = sorted({min(V8, w) for w in range(CCE_BWD_CHUNK // 2, top + 1, 256)})
-    return min(widths, key=lambda w: V // w * cost(w) + (cost(V % w) if V % w else 0))
-
-
+    """Vocabulary columns per chunk of the backward, by the estimated times of the products (``csrc/gemm.cu``).
+    Measured with a 151,936-word vocabulary, K = 896, forward + backward, chunks of 8192 columns -> chosen:
+    64 tokens 1311 -> 798 us, 512 1533 -> 1023, 2048 2740 -> 2150, 4096 3905 -> 3790, 8192 the same (8192 columns)."""
+    return _ext.lib().cb_cce_chunk(M, K, V, CCE_BWD_CHUNK, CCE_BWD_ELEMENTS, sms)
 
 
 class _LinearCEFn(torch.autograd.Function):

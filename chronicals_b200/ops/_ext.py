@@ -58,6 +58,7 @@ _PROTOTYPES = {
     "cb_gemm2sm_cost_ns": [I, I, I, I, I, I, I],
     "cb_gemm_choice": [I, I, I, I, I, I, I],
     "cb_glu_bwd_fused_pays": [I, I, I, I],
+    "cb_cce_chunk": [I, I, I, I, L, I],
     "cb_gemm2sm_bf16_dual": [P, P, P, P, P, P, P, I, I, I, I, L, L, L, L, L, L, I, P, P],
     "cb_gemm2sm_bf16_glu_bwd": [P, P, P, P, I, I, I, L, L, L, L, P, P],
     "cb_gemm2sm_bf16_glu": [P, P, P, P, P, I, I, I, L, L, L, L, P, P],
@@ -145,7 +146,7 @@ def lib() -> ctypes.CDLL:
 
 
 # device kernels launched by one call of each entry point (0: host-only query)
-_KERNELS_PER_CALL = {"cb_gemm2sm_supported": 0, "cb_gemm2sm_cost_ns": 0, "cb_gemm_choice": 0, "cb_glu_bwd_fused_pays": 0, "cb_cce_num_splits": 0, "cb_rmsnorm_max_n": 0, "cb_rmsnorm_bwd_blocks": 0, "cb_opt_chunk": 0,
+_KERNELS_PER_CALL = {"cb_gemm2sm_supported": 0, "cb_gemm2sm_cost_ns": 0, "cb_gemm_choice": 0, "cb_glu_bwd_fused_pays": 0, "cb_cce_chunk": 0, "cb_cce_num_splits": 0, "cb_rmsnorm_max_n": 0, "cb_rmsnorm_bwd_blocks": 0, "cb_opt_chunk": 0,
                      "cb_embedding_rank_max": 0, "cb_embedding_part_rows": 0, "cb_embedding_bwd": 2, "cb_cce_combine": 2, "cb_rmsnorm_bwd": 2, "cb_grad_clip_coef": 2, "cb_attn_bwd": 3}
 LAUNCH_COUNT = [0]
 

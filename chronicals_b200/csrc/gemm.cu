@@ -763,9 +763,11 @@ int pick_block_n(int M, int N, int forced) {
 // Which kernel: the estimate of the CTA-pair kernel (gemm2sm.cu) against those of the single-CTA kernels, fitted to 276 products
 // (four model sizes, 128 to 8192 tokens, forward, dgrad and wgrad): rounds of whole tiles over the SMs, a fixed cost that is
 // 2 us lower, and the output.  Returns 0 for pairs, else the single-CTA tile width.  A grid of 128-wide tiles that fits one
-// round is never widened: fewer CTAs would take longer for as many k-blocks (896 x 896 x 128: 5.0 us against 5.9 of 256; the
-// two estimates lie within the fit's error there).  Against the width that pads N least, whatever the rounds: 2.8 % less time
-// on average over those products, 32 % less at most (4096 x 1536 x 8960: 121 -> 83 us).
+// round runs as it is: wider tiles and pairs only make fewer CTAs take longer for as many k-blocks, and the estimates lie within
+// the fit's error there (896 x 896 x 128: 5.0 us against 5.9 of 256; 696 x 120 x 18,944: 68 against 77 of pairs; 32 x 9728 x 6000:
+// 30 against 33; pairs won by 4 % at most).  Outputs of an adapter's width have pair tiles of their own and are compared.
+// Against the width that pads N least, whatever the rounds: 2.8 % less time on average over those products, 32 % less at most
+// (4096 x 1536 x 8960: 121 -> 83 us).
 int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool pairs_possible, int sms, double* us = nullptr) {
   const bool mn = a_mn && b_mn;
   const double kb = (K + 63) / 64, mb = 1e-6 * M * N * out_bytes;
@@ -775,7 +777,8 @@ int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool p
   const double t256 = (mn ? 4.43 + 0.35 * r256 : 4.1) + (mn ? 0.382 : 0.358) * r256 * kb + 0.147 * mb;
   const bool narrow = r128 == 1 || t128 < t256;
   const double single = narrow ? t128 : t256;
-  const double pair = pairs_possible ? 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes, sms) : single + 1.0;
+  const bool compare = pairs_possible && (r128 > 1 || (N <= 64 && !a_mn));
+  const double pair = compare ? 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes, sms) : single + 1.0;
   if (us != nullptr) *us = std::min(single, pair);           // the estimate for the kernel that is taken
   return pair <= single ? 0 : narrow ? 128 : 256;
 }

@@ -4,9 +4,9 @@ import random
 from chronicals_b200.ops import _ext
 
 
-def test_one_round_of_narrow_tiles_is_not_widened():
+def test_one_round_of_narrow_tiles_runs_as_it_is():
     choice, rng = _ext.lib().cb_gemm_choice, random.Random(1)
-    sizes = [(896, 896, 128), (1152, 896, 128), (896, 896, 64), (1, 1, 8), (128, 148 * 128, 64)]
+    sizes = [(896, 896, 128), (1152, 896, 128), (896, 896, 64), (1, 1, 8), (128, 148 * 128, 64), (696, 120, 18944), (32, 9728, 6000)]
     sizes += [tuple(int(2 ** rng.uniform(3, 14)) for _ in range(3)) for _ in range(3000)]
     seen = set()
     for M, N, K in sizes:
@@ -14,7 +14,7 @@ def test_one_round_of_narrow_tiles_is_not_widened():
             got = choice(M, N, K, a_mn, b_mn, 2, 148)
             seen.add(got)
             if -(-M // 128) * -(-N // 128) <= 148:
-                assert got != 256, (M, N, K)
+                assert got == 128 or (got == 0 and N <= 64 and not a_mn), (M, N, K)      # an adapter's pair tiles
     assert seen == {0, 128, 256}
 
 

@@ -995,13 +995,12 @@ extern "C" {
 
 // Vocabulary columns per chunk of the fused linear-cross-entropy's backward (whole 256-column tiles, or all of V rounded up to 8),
 // with at most max(elements, M * base) values of d(logits) in a chunk.  A chunk is three products, d(logits), dH and dW_c, and
-// costs what the dispatch estimates for them; few wide chunks save launches, fills and drains, and a width is good that fills the
-// last round of dW's tiles.  So the widths looked at are equal shares of V, the fewest that the bound allows and two more, and
-// the widest that fill whole rounds of one of the three tile widths of the pair kernel: at most 13, a few microseconds.
+// costs what the dispatch estimates for them; few wide chunks save launches, fills and drains.  So the widths looked at are equal
+// shares of V: the fewest that the bound allows, and one and two more, in which the products' tiles may fill their rounds better.
 // `base` stays unless another width is estimated 8 % faster, which is how far the estimates are off (6000 tokens, K = 3584:
 // 9472 columns, estimated 7 % faster, took 20.6 ms against 19.7).  Times by size: ops._cce_chunk.
 int cb_cce_chunk(int M, int K, int V, int base, long long elements, int sms) {
-  if (M <= 0 || K <= 0 || V <= 0 || base < 256 || sms < 2) return -1;
+  if (M <= 0 || K <= 0 || V <= 0 || base <= 0 || sms < 2) return -1;
   const long long all = (V + 7LL) / 8 * 8;
   const long long top = std::min(all, std::max<long long>(base, elements / M / 256 * 256));
   const auto product = [&](long long m, long long n, long long k, int a_mn, int out_bytes) {
@@ -1017,18 +1016,14 @@ int cb_cce_chunk(int M, int K, int V, int base, long long elements, int sms) {
   const auto whole = [&](long long w) { return static_cast<double>(V / w) * chunk(w) + (V % w ? chunk(V % w) : 0.0); };
   long long best = std::min<long long>(all, base);
   double best_us = 0.92 * whole(best);
-  const auto look_at = [&](long long w) {
-    if (w < std::min<long long>(all, base / 2) || w > top) return;
-    const double us = whole(w);
+  const long long fewest = (all + top - 1) / top;
+  for (long long n = fewest; n < fewest + 3; ++n) {
+    const long long w = std::min(all, ((all + n - 1) / n + 255) / 256 * 256);
+    const double us = w <= top ? whole(w) : best_us;
     if (us < best_us) {
       best_us = us;
       best = w;
     }
-  };
-  for (long long n = (all + top - 1) / top, i = 0; i < 3; ++i, ++n) look_at(std::min(all, ((all + n - 1) / n + 255) / 256 * 256));
-  for (int bn = 256; bn >= 192; bn -= 32) {
-    const long long across = (K + bn - 1) / bn, rounds = top / 256 * across / (sms / 2);
-    for (long long r = rounds; r > 0 && r > rounds - 3; --r) look_at(sms / 2 * r / across * 256);
   }
   return static_cast<int>(best);
 }

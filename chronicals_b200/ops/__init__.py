@@ -704,7 +704,7 @@ CCE_BWD_ELEMENTS = 8192 * 8192     # ... and how many values that is: fewer toke
 def _cce_chunk(M: int, K: int, V: int, sms: int) -> int:
     """Vocabulary columns per chunk of the backward, by the estimated times of the products (``csrc/gemm.cu``).
     Measured with a 151,936-word vocabulary, K = 896, forward + backward, chunks of 8192 columns -> chosen:
-    64 tokens 1311 -> 798 us, 512 1533 -> 1023, 2048 2740 -> 2150, 4096 3905 -> 3790, 8192 the same (8192 columns)."""
+    64 tokens 1315 -> 802 us, 512 1536 -> 1046, 2048 2748 -> 2152, 4096 3891 -> 3749, 8192 the same (8192 columns)."""
     return _ext.lib().cb_cce_chunk(M, K, V, CCE_BWD_CHUNK, CCE_BWD_ELEMENTS, sms)
 
 

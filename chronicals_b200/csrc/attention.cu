@@ -1312,7 +1312,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // dQ tile (fp32) -> shared memory as [128 x 32] boxes in the layout of the dq_acc tensor map -> one TMA
       // reduce-add per box instead of eight red.global.add per thread and box.  The boxes go to the P / dS buffer,
       // which nobody reads any more.
-      // Rows past the end of the document carry exact zeros (their P was masked), rows past T are clipped.
+      // Rows past the end of the document carry exact zeros (P is zero there, K and V are this document's and its neighbour's
+      // and have to be finite), rows past T are clipped.
 #pragma unroll
       for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
         uint32_t dq[32];
@@ -1377,13 +1378,13 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Backward, pipelined form (D = 128, and D = 64 with few or long blocks).  One CTA: kv block `jb` of one document, one query head; loops over the query
-// blocks i >= jb.  The scores are kept transposed (rows = keys, S^T = K Q^T), so that P^T is an A operand straight from
+// Backward, pipelined form (D = 128, and D = 64 with few or long blocks).  One CTA: kv block `jb` of one document, one query
+// head; loops over the query blocks i >= jb.  The scores are kept transposed (rows = keys, S^T = K Q^T), so that P^T is an A operand straight from
 // TMEM and dS^T, written to shared memory once, serves as the K-major A operand of dK and as the MN-major one of dQ:
 //   S^T = K Q^T -> P^T -> dV += P^T dO;   dP^T = V dO^T -> dS^T -> dQ = dS K, dK += dS^T Q
 // At D = 128 the five products of an iteration read 288 KB of operands from shared memory and the rest moves 224 KB:
-// 4096 cycles at 128 bytes a cycle, against 2560 of the tensor core.  One phase after another (the form above, which D =
-// 128 used before) took 10,500; here the roles work on different products at the same time, each in its own warps:
+// 4096 cycles at 128 bytes a cycle, against 2560 of the tensor core.  One phase after another, as in the form above, takes
+// 10,500; here the roles work on different products at the same time, each in its own warps:
 //   warps 0-7   P and dS: warps w and w + 4 share 32 keys and take 64 query columns each
 //   warps 8-11  dQ out of TMEM, 32 query rows each: all of it to registers at once, so that dP may follow, then through
 //               two 4 KB boxes a warp and TMA reduce-add
@@ -1392,6 +1393,10 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 //   warp 13     TMA loads (Q two blocks deep, dO one) and the statistics of the query rows
 // TMEM: S^T [0, 128) with P^T over the first half of each 32 columns, dP^T [128, 256), dV, dK, and dQ over dP^T (D = 128)
 // or in columns of its own (D = 64, where dP need not wait for dQ to leave).
+// A document's last query block brings rows of the next one with it.  Their probabilities are exact zeros, which keeps them
+// out of dV and dK as long as their Q and dO are finite: 0 x NaN and 0 x inf are NaN, in this form as in the one above (and
+// so it is with the V rows of the next document in the forward pass).  What this form writes to a neighbour's rows is
+// zero whatever either document holds.
 // What bounds it now: 6600 cycles an iteration, of which the products with the waits between the roles take 5900 and the
 // softmax with them 5200 when the other is left out; the reduce-adds of dQ cost 60 us of 720.
 // Measured (kernel alone): 2 x 4096 tokens, 28 / 4 heads of 128: 1144 -> 721 us (526 -> 834 TFLOP/s); 27 documents in 8192
@@ -1544,7 +1549,7 @@ attn_bwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             for (int p = 0; p < PANELS; ++p) tma_load_2d(sV + p * 16384, &tmV, v_full, hkv * D + p * 64, row0);
           }
         }
-        // rows past the end of the document get lse = +inf: their probabilities are exact zeros
+        // rows past the end of the document get lse = +inf: finite scores give probabilities of exactly zero
   #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const bool in = (u_jb + it) * 128 + lane + 32 * k < len;
@@ -1645,7 +1650,7 @@ attn_bwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     for (int it = 0; it < n_it; ++it) {
       if (!wait_w(dq_full, it, CB_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
-uint32_t dq[D / 32][32];
+      uint32_t dq[D / 32][32];
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) tmem_ld_32x32(t_row + C_DQ + c * 32, dq[c]);
       tmem_ld_wait();

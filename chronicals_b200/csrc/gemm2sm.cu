@@ -785,8 +785,8 @@ int dispatch_layout(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap
 // What a product takes on CTA pairs with tiles of 256 x bn, in microseconds at full clock: whole tiles, ceil(T / pairs)
 // rounds of them; or cut along K, T / pairs rounds and the fixups (partial sums through L2, the last arrival's read-back:
 // 24 us, so only a long K and a mostly empty last round pay).  Fitted to 276 products (four model sizes, 128 to 8192
-// tokens, forward, dgrad and wgrad; 7 to 10 % off on average).  Of two widths the one that pads N least used to be taken,
-// whatever the rounds: 4096 x 1536 x 8960 ran two rounds of 256 (121 us) where two of 192 take 83.
+// tokens, forward, dgrad and wgrad; 7 to 10 % off on average).  The width that pads N least is no guide: at 4096 x 1536 x 8960
+// two rounds of 256 take 121 us and two of 192 take 83.
 struct PairPlan {
   int bn;
   bool split;

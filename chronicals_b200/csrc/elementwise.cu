@@ -543,16 +543,21 @@ embedding_rank_fill_kernel(const long long* __restrict__ ids, int* __restrict__ 
 // step 3, against 292 us with a block per run.
 constexpr int EMB_CHUNK = 32;
 
+// Index type I: int as step 1 leaves them, long long as the library's sort does.
+template <typename I>
+__device__ __forceinline__ int emb_row(I id, long long V) { return id >= 0 && id < V ? static_cast<int>(id) : EMB_NO_ROW; }
+
+template <typename I>
 __global__ void __launch_bounds__(128)
-embedding_bwd_kernel(const int* __restrict__ sorted_ids, const int* __restrict__ perm, const bf16* __restrict__ dout,
-                     bf16* __restrict__ dtable, float* __restrict__ part, int T, int N) {
+embedding_bwd_kernel(const I* __restrict__ sorted_ids, const I* __restrict__ perm, const bf16* __restrict__ dout,
+                     bf16* __restrict__ dtable, float* __restrict__ part, int T, int N, long long V) {
   __shared__ int sid[EMB_CHUNK + 2], src[EMB_CHUNK];   // sid[k + 1] = id of the chunk's k-th token, with both neighbours
   const int r0 = blockIdx.x * EMB_CHUNK;
   const int n = T - r0 < EMB_CHUNK ? T - r0 : EMB_CHUNK;
   for (int k = threadIdx.x; k < EMB_CHUNK + 2; k += blockDim.x) {
     const int r = r0 + k - 1;
-    sid[k] = r >= 0 && r < T ? sorted_ids[r] : -1;
-    if (k >= 1 && k <= n) src[k - 1] = perm[r];
+    sid[k] = r >= 0 && r < T ? emb_row(sorted_ids[r], V) : -1;
+    if (k >= 1 && k <= n) src[k - 1] = static_cast<int>(perm[r]);
   }
   __syncthreads();
   const int v = blockIdx.y * blockDim.x + threadIdx.x;
@@ -593,12 +598,14 @@ embedding_bwd_kernel(const int* __restrict__ sorted_ids, const int* __restrict__
 
 // Step 3: the block of the chunk in which a run begins that its last token does not end adds the parts of the chunks
 // that follow, in their order, and writes the row.
+template <typename I>
 __global__ void __launch_bounds__(128)
-embedding_bwd_span_kernel(const int* __restrict__ sorted_ids, bf16* __restrict__ dtable, const float* __restrict__ part, int T, int N) {
+embedding_bwd_span_kernel(const I* __restrict__ sorted_ids, bf16* __restrict__ dtable, const float* __restrict__ part, int T, int N,
+                          long long V) {
   const int r0 = blockIdx.x * EMB_CHUNK, last = r0 + EMB_CHUNK - 1;
   if (last + 1 >= T) return;
-  const int id = sorted_ids[last];
-  if (id == EMB_NO_ROW || sorted_ids[last + 1] != id) return;
+  const I id = sorted_ids[last];
+  if (emb_row(id, V) == EMB_NO_ROW || sorted_ids[last + 1] != id) return;
   if (r0 > 0 && sorted_ids[r0] == id && sorted_ids[r0 - 1] == id) return;     // began before this chunk
   const int v = blockIdx.y * blockDim.x + threadIdx.x;
   if (v >= N / 8) return;
@@ -923,6 +930,9 @@ int ce_split(long long rows, int V) {
   return split;
 }
 // Layout of a row of N columns (see RowLayout): vectors a thread, threads a block, rows a block; vpl = 0: too wide
+// Two vectors a thread end at 320 threads, where registers and the ring still let an SM hold two blocks of the backward; built
+// for 512 threads (64 registers, one block an SM) they take longer than four vectors and a ring of two (backward, 16,384 rows:
+// 5376 columns 179 against 134 us, 8192 217 against 169; forward 66 / 61 and 90 / 87).
 struct RowPlan {
   int vpl, threads, rows;
 };
@@ -1102,8 +1112,10 @@ int cb_embedding_fwd(const long long* ids, const void* table, void* out, long lo
   return static_cast<int>(cudaGetLastError());
 }
 
-// Most tokens that cb_embedding_rank_fill sorts itself; more of them are sorted by the caller.
-int cb_embedding_rank_max() { return 32768; }
+// Most tokens that cb_embedding_rank_fill sorts itself; more of them are sorted by the caller.  Counting grows with the square
+// of the tokens (counting / the library's sort, whole backward: 8192 tokens, 32,000 x 896: 56 / 128 us, 20,480 124 / 138, 22,528
+// 134 / 140, 24,576 175 / 142, 32,768 267 / 150; 500 x 256: 22,528 122 / 122, 24,576 130 / 122).
+int cb_embedding_rank_max() { return 22528; }
 
 // Zeroes dtable [V, N] and, with sorted_ids / perm given (T int32 each), sorts the T ids (stable).
 int cb_embedding_rank_fill(const long long* ids, int* sorted_ids, int* perm, void* dtable, long long T, int N, long long V,
@@ -1121,17 +1133,21 @@ int cb_embedding_rank_fill(const long long* ids, int* sorted_ids, int* perm, voi
 // Rows of N floats that `part` of cb_embedding_bwd holds for T tokens.
 int cb_embedding_part_rows(long long T) { return static_cast<int>(2 * ((T + cb::EMB_CHUNK - 1) / cb::EMB_CHUNK)); }
 
-// dtable (zeroed) receives the sums of the rows of dout [T, N] over equal ids; sorted_ids ascending (ids that are no row
-// of the table hold 0x7ffffffe), perm the source token of each.
-int cb_embedding_bwd(const int* sorted_ids, const int* perm, const void* dout, void* dtable, float* part, long long T, int N,
-                     void* stream) {
-  if (N % 8 != 0 || T <= 0 || T > 0x7fffff00LL) return -1;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
+// dtable [V, N] (zeroed) receives the sums of the rows of dout [T, N] over equal ids; sorted_ids ascending (ids outside [0, V)
+// are no row of the table), perm the source token of each; both int32, or int64 with `wide`.
+int cb_embedding_bwd(const void* sorted_ids, const void* perm, const void* dout, void* dtable, float* part, long long T, int N,
+                     long long V, int wide, void* stream) {
+  if (N % 8 != 0 || T <= 0 || T > 0x7fffff00LL || V <= 0 || V >= cb::EMB_NO_ROW) return -1;
   const dim3 grid(static_cast<unsigned>((T + cb::EMB_CHUNK - 1) / cb::EMB_CHUNK), (N / 8 + 127) / 128);
-  cb::embedding_bwd_kernel<<<grid, 128, 0, s>>>(sorted_ids, perm, static_cast<const cb::bf16*>(dout), static_cast<cb::bf16*>(dtable),
-                                                part, static_cast<int>(T), N);
-  cb::embedding_bwd_span_kernel<<<grid, 128, 0, s>>>(sorted_ids, static_cast<cb::bf16*>(dtable), part, static_cast<int>(T), N);
-  return static_cast<int>(cudaGetLastError());
+  const auto go = [&](const auto* ids, const auto* from) {
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    cb::bf16* out = static_cast<cb::bf16*>(dtable);
+    cb::embedding_bwd_kernel<<<grid, 128, 0, s>>>(ids, from, static_cast<const cb::bf16*>(dout), out, part, static_cast<int>(T), N, V);
+    cb::embedding_bwd_span_kernel<<<grid, 128, 0, s>>>(ids, out, part, static_cast<int>(T), N, V);
+    return static_cast<int>(cudaGetLastError());
+  };
+  if (wide) return go(static_cast<const long long*>(sorted_ids), static_cast<const long long*>(perm));
+  return go(static_cast<const int*>(sorted_ids), static_cast<const int*>(perm));
 }
 
 int cb_ce_logits(const void* logits, const long long* labels, long long rows, long long ld, int V, int is_bf16,

@@ -653,15 +653,14 @@ class _EmbeddingFn(torch.autograd.Function):
         if own:
             order = torch.empty(2, T, dtype=torch.int32, device=dout.device)
             sorted_ids, perm = order[0], order[1]
-        else:                                          # counting against every other id no longer hides behind the zero fill
-            s64, p64 = torch.sort(torch.where((flat >= 0) & (flat < V), flat, 0x7ffffffe), stable=True)
-            sorted_ids, perm = s64.int(), p64.int()
+        else:                                          # counting against every other id takes longer than sorting them
+            sorted_ids, perm = torch.sort(flat, stable=True)
         code = L.cb_embedding_rank_fill(flat.data_ptr(), sorted_ids.data_ptr() if own else None, perm.data_ptr() if own else None,
                                         dtable.data_ptr(), T, N, V, _ext.stream_ptr())
         _ext.check(code, "embedding_rank_fill")
         part = torch.empty(L.cb_embedding_part_rows(T) * N, dtype=torch.float32, device=dout.device)
         code = L.cb_embedding_bwd(sorted_ids.data_ptr(), perm.data_ptr(), d2.data_ptr(), dtable.data_ptr(), part.data_ptr(),
-                                  T, N, _ext.stream_ptr())
+                                  T, N, V, int(not own), _ext.stream_ptr())
         _ext.check(code, "embedding_bwd")
         return None, dtable
 

@@ -47,7 +47,7 @@ _PROTOTYPES = {
     "cb_embedding_rank_max": [],
     "cb_embedding_part_rows": [L],
     "cb_embedding_rank_fill": [P, P, P, P, L, I, L, P],
-    "cb_embedding_bwd": [P, P, P, P, P, L, I, P],
+    "cb_embedding_bwd": [P, P, P, P, P, L, I, L, I, P],
     "cb_ce_logits": [P, P, L, L, I, I, L, F, F, P, P, P],
     "cb_ce_logits_grad": [P, P, P, P, P, P, L, L, L, I, I, L, F, F, P],
     "cb_attn_fwd": [P, P, P, P, P, P, I, I, I, I, I, L, L, L, L, F, P, P],

@@ -762,12 +762,15 @@ int pick_block_n(int M, int N, int forced) {
 
 // Which kernel: the estimate of the CTA-pair kernel (gemm2sm.cu) against those of the single-CTA kernels, fitted to 276 products
 // (four model sizes, 128 to 8192 tokens, forward, dgrad and wgrad): rounds of whole tiles over the SMs, a fixed cost that is
-// 2 us lower, and the output.  Returns 0 for pairs, else the single-CTA tile width.  A grid of 128-wide tiles that fits one
-// round runs as it is: wider tiles and pairs only make fewer CTAs take longer for as many k-blocks, and the estimates lie within
-// the fit's error there (896 x 896 x 128: 5.0 us against 5.9 of 256; 696 x 120 x 18,944: 68 against 77 of pairs; 32 x 9728 x 6000:
-// 30 against 33; pairs won by 4 % at most).  Outputs of an adapter's width have pair tiles of their own and are compared.
-// Against the width that pads N least, whatever the rounds: 2.8 % less time on average over those products, 32 % less at most
-// (4096 x 1536 x 8960: 121 -> 83 us).
+// 2 us lower, and the output.  Returns 0 for pairs, else the single-CTA tile width.
+// The estimates do not decide where the 128-wide tiles fit one round: wider single-CTA tiles only make fewer CTAs take longer
+// for as many k-blocks (896 x 896 x 128: 5.0 us against 5.9), and CTA pairs, 192 wide, win with both operands K-major, a long K
+// and rows enough for both CTAs or few columns, where they read less a product (2048 x 1152 x 18,944: 76 / 86, 128 x 552 x 8960:
+// 36 / 39), and lose elsewhere (128 x 9728 x 8960: 45 / 42, 2048 x 1152 x 3584 with B as [K, N]: more at every size below 18,944).
+// Over 720 products of one round this takes 0.1 % more than the better of the two each time.  Outputs of an adapter's width have
+// pair tiles of their own and are compared.
+// Against the width that pads N least, whatever the rounds: 2.8 % less time on average over the products of the fit, 32 % less
+// at most (4096 x 1536 x 8960: 121 -> 83 us).
 int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool pairs_possible, int sms, double* us = nullptr) {
   const bool mn = a_mn && b_mn;
   const double kb = (K + 63) / 64, mb = 1e-6 * M * N * out_bytes;
@@ -777,10 +780,14 @@ int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool p
   const double t256 = (mn ? 4.43 + 0.35 * r256 : 4.1) + (mn ? 0.382 : 0.358) * r256 * kb + 0.147 * mb;
   const bool narrow = r128 == 1 || t128 < t256;
   const double single = narrow ? t128 : t256;
-  const bool compare = pairs_possible && (r128 > 1 || (N <= 64 && !a_mn));
-  const double pair = compare ? 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes, sms) : single + 1.0;
-  if (us != nullptr) *us = std::min(single, pair);           // the estimate for the kernel that is taken
-  return pair <= single ? 0 : narrow ? 128 : 256;
+  const bool adapter = N <= 64 && !a_mn;
+  const bool long_k = r128 == 1 && !adapter && !a_mn && !b_mn && kb >= 72 && (M > 256 || N <= 1024) &&
+                      static_cast<long long>((M + 255) / 256) * ((N + 191) / 192) <= sms / 2;
+  const bool compare = pairs_possible && (r128 > 1 || adapter || long_k);
+  const double pair = compare ? 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes, sms) : 0.0;
+  const bool pairs = compare && (long_k || pair <= single);
+  if (us != nullptr) *us = pairs ? pair : single;            // the estimate for the kernel that is taken
+  return pairs ? 0 : narrow ? 128 : 256;
 }
 
 // Tensor map of the output for the staged epilogue; returns 0 and sets *ok when C qualifies

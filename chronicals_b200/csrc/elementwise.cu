@@ -660,6 +660,14 @@ __device__ __forceinline__ int ce_head(const T* p, int V) {
   return h < V ? h : V;
 }
 
+template <int N>
+__device__ __forceinline__ float ce_max(const uint4& u) {
+  if (N == 4) return fmaxf(fmaxf(__uint_as_float(u.x), __uint_as_float(u.y)), fmaxf(__uint_as_float(u.z), __uint_as_float(u.w)));
+  const bf162* h = reinterpret_cast<const bf162*>(&u);
+  const float2 f = __bfloat1622float2(__hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+  return fmaxf(f.x, f.y);
+}
+
 // running (max, sum of exp(v - max)); an all -inf prefix keeps the sum at 0, NaN stays NaN
 struct CeAcc {
   float m = -INFINITY, s = 0.f, sum = 0.f;
@@ -670,21 +678,35 @@ struct CeAcc {
     m = nm;
     sum += osum;
   }
-  template <int K>
-  __device__ __forceinline__ void add(const float (&v)[K]) {
-    float vm = v[0];
+  __device__ __forceinline__ void add(float v) {
+    const float nm = fmaxf(m, v), b = base(nm);
+    s = s * __expf(m - b) + __expf(v - b);
+    m = nm;
+    sum += v;
+  }
+  // packed vectors of N values, those that are `in` the row; the maximum of bf16 values is taken in pairs, before they are
+  // unpacked: held unpacked, a batch of 32 takes 62 registers and leaves an SM half the blocks
+  template <int N>
+  __device__ __forceinline__ void add(const uint4 (&u)[CE_BATCH], const bool (&in)[CE_BATCH]) {
+    float nm = m;
 #pragma unroll
-    for (int i = 1; i < K; ++i) vm = fmaxf(vm, v[i]);
-    const float nm = fmaxf(m, vm), b = base(nm);
-    float e = 0.f, t = 0.f;
+    for (int i = 0; i < CE_BATCH; ++i)
+      if (in[i]) nm = fmaxf(nm, ce_max<N>(u[i]));
+    const float b = base(nm);
+    float e = 0.f;
 #pragma unroll
-    for (int i = 0; i < K; ++i) {
-      e += __expf(v[i] - b);
-      t += v[i];
-    }
+    for (int i = 0; i < CE_BATCH; ++i)
+      if (in[i]) {
+        float w[N];
+        ce_unpack(u[i], w);
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          e += __expf(w[j] - b);
+          sum += w[j];
+        }
+      }
     s = s * __expf(m - b) + e;
     m = nm;
-    sum += t;
   }
 };
 
@@ -713,38 +735,31 @@ ce_logits_kernel(const T* __restrict__ logits, const long long* __restrict__ lab
   const T* lp = logits + row * ld;
   const int head = ce_head(lp, V), nvec = (V - head) / N, tail0 = head + nvec * N;
   const uint4* vp = reinterpret_cast<const uint4*>(lp + head);
-  const int step = EW_THREADS * gridDim.y;
+  const int step = blockDim.x * gridDim.y;
   CeAcc a;
-  int c = blockIdx.y * EW_THREADS + threadIdx.x;
-  for (; c + (CE_BATCH - 1) * step < nvec; c += CE_BATCH * step) {
-    uint4 u[CE_BATCH];
+  int c = blockIdx.y * blockDim.x + threadIdx.x;
+  uint4 u[CE_BATCH];
+  if (nvec > CE_BATCH * step) {                        // (a row of one batch goes the second way with all its threads)
+    const bool all[CE_BATCH] = {true, true, true, true};
+    for (; c + (CE_BATCH - 1) * step < nvec; c += CE_BATCH * step) {
 #pragma unroll
-    for (int i = 0; i < CE_BATCH; ++i) u[i] = vp[c + i * step];
-    float v[CE_BATCH * N];
+      for (int i = 0; i < CE_BATCH; ++i) u[i] = vp[c + i * step];
+      a.add<N>(u, all);
+    }
+  }
+  if (c < nvec) {                                      // a batch that need not be full
+    bool in[CE_BATCH];
 #pragma unroll
     for (int i = 0; i < CE_BATCH; ++i) {
-      float w[N];
-      ce_unpack(u[i], w);
-#pragma unroll
-      for (int j = 0; j < N; ++j) v[i * N + j] = w[j];
+      in[i] = c + i * step < nvec;
+      if (in[i]) u[i] = vp[c + i * step];
     }
-    a.add(v);
-  }
-  for (; c < nvec; c += step) {
-    float w[N];
-    ce_unpack(vp[c], w);
-    a.add(w);
+    a.add<N>(u, in);
   }
   if (blockIdx.y == 0) {                               // at most N - 1 values at either end
     const int t = static_cast<int>(threadIdx.x);
-    if (t < head) {
-      const float w[1] = {ldf(lp + t)};
-      a.add(w);
-    }
-    if (tail0 + t < V) {
-      const float w[1] = {ldf(lp + tail0 + t)};
-      a.add(w);
-    }
+    if (t < head) a.add(ldf(lp + t));
+    if (tail0 + t < V) a.add(ldf(lp + tail0 + t));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -759,7 +774,7 @@ ce_logits_kernel(const T* __restrict__ logits, const long long* __restrict__ lab
   __syncthreads();
   if (threadIdx.x == 0) {
     a = CeAcc();
-    for (int i = 0; i < EW_THREADS / 32; ++i) a.merge(sm[i], ss[i], sl[i]);
+    for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) a.merge(sm[i], ss[i], sl[i]);
   }
   if (gridDim.y > 1) {
     cl.barrier_wait(std::move(started));
@@ -797,14 +812,22 @@ ce_logits_grad_kernel(const T* logits, T* dlogits, const long long* __restrict__
   const bool valid = lab != ignore_index && lab >= 0 && lab < V;
   const T* lp = logits + row * ld;
   T* dp = dlogits + row * ldd;
+  const int at = valid ? static_cast<int>(lab) : -1;
   const float lse = lse_in[row];
   const float gs = valid ? gscale[row] * gout[0] : 0.f;
   const float coef = 1.f + 2.f * z_weight * lse;
   const float smv = smoothing / static_cast<float>(V);
   const float hit = 1.f - smoothing;
+  // bf16 results: the constants of the row are folded into two multiply-adds a value (error 1e-6, far below the rounding)
+  constexpr float LOG2E_F = 1.4426950408889634f;
+  const float lse2 = lse * LOG2E_F, coef_gs = coef * gs, smv_gs = smv * gs, hit_gs = hit * gs;
   const auto grad = [&](float v, int c) {
+    if (sizeof(T) == 2) {
+      const float p = fmaf(ex2_approx(fmaf(v, LOG2E_F, -lse2)), coef_gs, -smv_gs);
+      return c == at ? p - hit_gs : p;
+    }
     float p = __expf(v - lse) * coef - smv;
-    if (c == lab) p -= hit;
+    if (c == at) p -= hit;
     return p * gs;
   };
   // source and destination rows may start at different distances from a 16-byte boundary: value by value then
@@ -812,34 +835,29 @@ ce_logits_grad_kernel(const T* logits, T* dlogits, const long long* __restrict__
   const int head = vec ? ce_head(lp, V) : V, nvec = (V - head) / N, tail0 = head + nvec * N;
   const uint4* vp = reinterpret_cast<const uint4*>(lp + head);
   uint4* wp = reinterpret_cast<uint4*>(dp + head);
-  const int step = EW_THREADS * gridDim.y;
-  const int first = blockIdx.y * EW_THREADS + threadIdx.x;
+  const int step = blockDim.x * gridDim.y;
+  const int first = blockIdx.y * blockDim.x + threadIdx.x;
   if (!valid) {
     for (int c = first; c < nvec; c += step) wp[c] = make_uint4(0u, 0u, 0u, 0u);
     for (int c = first; c < head; c += step) stf(dp + c, 0.f);
     for (int c = tail0 + first; c < V; c += step) stf(dp + c, 0.f);
     return;
   }
-  int c = first;
-  for (; c + (CE_BATCH - 1) * step < nvec; c += CE_BATCH * step) {
+  const auto put = [&](const uint4& u, int v) {
+    float w[N];
+    ce_unpack(u, w);
+#pragma unroll
+    for (int j = 0; j < N; ++j) w[j] = grad(w[j], head + v * N + j);
+    wp[v] = ce_pack(w);
+  };
+  for (int c = first; c < nvec; c += CE_BATCH * step) {
     uint4 u[CE_BATCH];
 #pragma unroll
-    for (int i = 0; i < CE_BATCH; ++i) u[i] = vp[c + i * step];
+    for (int i = 0; i < CE_BATCH; ++i)
+      if (c + i * step < nvec) u[i] = vp[c + i * step];
 #pragma unroll
-    for (int i = 0; i < CE_BATCH; ++i) {
-      float w[N];
-      ce_unpack(u[i], w);
-#pragma unroll
-      for (int j = 0; j < N; ++j) w[j] = grad(w[j], head + (c + i * step) * N + j);
-      wp[c + i * step] = ce_pack(w);
-    }
-  }
-  for (; c < nvec; c += step) {
-    float w[N];
-    ce_unpack(vp[c], w);
-#pragma unroll
-    for (int j = 0; j < N; ++j) w[j] = grad(w[j], head + c * N + j);
-    wp[c] = ce_pack(w);
+    for (int i = 0; i < CE_BATCH; ++i)
+      if (c + i * step < nvec) put(u[i], c + i * step);
   }
   for (int i = first; i < head; i += step) stf(dp + i, grad(ldf(lp + i), i));
   for (int i = tail0 + first; i < V; i += step) stf(dp + i, grad(ldf(lp + i), i));
@@ -922,12 +940,31 @@ int grid_for(long long work_items, int per_block, int max_waves = 8) {
   if (b < 1) b = 1;
   return static_cast<int>(b);
 }
-// Blocks that share one row of logits.  One is enough once the rows alone fill the chip (four blocks an SM); with
-// fewer, a row is cut in 2, 4 or 8 (a portable cluster) as long as every piece keeps 4096 values.
+// Blocks that share one row of logits.  In the gradient, one is enough once the rows alone fill the chip (four blocks an SM); with
+// fewer, a row is cut in 2, 4 or 8 as long as every piece keeps 4096 values.
 int ce_split(long long rows, int V) {
   int split = 1;
   while (split < 8 && rows * split < 4LL * sm_count() && V / (2 * split) >= 4096) split *= 2;
   return split;
+}
+// In the forward pass, where a row is `nvec` 16-byte vectors, they form a cluster (a portable one has 8 at most) and meeting costs it about a microsecond:
+// long rows as above in pieces of 2048 vectors, or rows so few that they leave half the SMs without a block.  Measured, bf16,
+// one / two / four blocks a row: 16 x 32,000 6.2 / 5.4 / 4.4 us, 200 x 50,257 (one: 11 and more) 9.7 / 10.4, 400 x 16,384 6.3 / 8.1,
+// 100 x 8192 3.5 / 4.4.
+int ce_cluster(long long rows, int nvec) {
+  int split = 1;
+  while (split < 8 && ((rows * split < 4LL * sm_count() && nvec / (2 * split) >= 2048) ||
+                       (2 * rows * split <= sm_count() && nvec >= 3072 && nvec / (2 * split) >= 512)))
+    split *= 2;
+  return split;
+}
+// Threads of a block of a row of logits: with rows enough to fill the chip (four blocks an SM) as many as have a whole batch of
+// vectors each, since a block of 256 for a row of a few kilobytes spends most of its time on reductions between threads without
+// data (20,000 x 1000 bf16: forward 58 us with 256 threads, 22 with 32); with fewer rows, a thread a vector.
+int ce_threads(long long rows, int V, int is_bf16) {
+  const int nvec = V / (is_bf16 ? 8 : 4) + 1, each = rows > 4LL * sm_count() ? cb::CE_BATCH : 1;
+  const int t = ((nvec + each - 1) / each + 31) / 32 * 32;
+  return t < cb::EW_THREADS ? t : cb::EW_THREADS;
 }
 // Layout of a row of N columns (see RowLayout): vectors a thread, threads a block, rows a block; vpl = 0: too wide
 // Two vectors a thread end at 320 threads, where registers and the ring still let an SM hold two blocks of the backward; built
@@ -1155,9 +1192,9 @@ int cb_ce_logits(const void* logits, const long long* labels, long long rows, lo
   if (rows <= 0) return -1;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
-  const int split = ce_split(rows, V);
+  const int split = ce_cluster(rows, V / (is_bf16 ? 8 : 4));
   cfg.gridDim = dim3(static_cast<unsigned>(rows), split);
-  cfg.blockDim = dim3(cb::EW_THREADS);
+  cfg.blockDim = dim3(ce_threads(rows, V, is_bf16));
   cfg.stream = static_cast<cudaStream_t>(stream);
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1;
@@ -1179,8 +1216,8 @@ int cb_ce_logits_grad(const void* logits, void* dlogits, const long long* labels
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (rows <= 0) return -1;
   const dim3 grid(static_cast<unsigned>(rows), ce_split(rows, V));
-  if (is_bf16) cb::ce_logits_grad_kernel<cb::bf16><<<grid, cb::EW_THREADS, 0, s>>>(static_cast<const cb::bf16*>(logits), static_cast<cb::bf16*>(dlogits), labels, lse, gscale, gout, ld, ldd, V, ignore_index, smoothing, z_weight);
-  else cb::ce_logits_grad_kernel<float><<<grid, cb::EW_THREADS, 0, s>>>(static_cast<const float*>(logits), static_cast<float*>(dlogits), labels, lse, gscale, gout, ld, ldd, V, ignore_index, smoothing, z_weight);
+  if (is_bf16) cb::ce_logits_grad_kernel<cb::bf16><<<grid, ce_threads(rows, V, 1), 0, s>>>(static_cast<const cb::bf16*>(logits), static_cast<cb::bf16*>(dlogits), labels, lse, gscale, gout, ld, ldd, V, ignore_index, smoothing, z_weight);
+  else cb::ce_logits_grad_kernel<float><<<grid, ce_threads(rows, V, 0), 0, s>>>(static_cast<const float*>(logits), static_cast<float*>(dlogits), labels, lse, gscale, gout, ld, ldd, V, ignore_index, smoothing, z_weight);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -48,6 +48,16 @@ def test_logits_cross_entropy_rows(rows, V, gap, shift, dtype):
         assert torch.equal(buf[shift:].view(rows, V + gap)[:, :V], lg)
 
 
+# a warp, two and eight a row with a batch that is just full, short of it and past it; rows on either side of the line between
+# one vector and four a thread; rows shared by clusters in pieces of either kind
+@pytest.mark.parametrize("rows,V,gap,shift", [(593, 128, 0, 0), (592, 1023, 1, 1), (593, 1023, 1, 1), (593, 1024, 0, 0), (600, 1025, 0, 0),
+                                              (593, 8192, 0, 0), (593, 8200, 0, 0), (40, 24576, 0, 0), (74, 24584, 0, 0),
+                                              (75, 24584, 0, 0), (300, 33001, 0, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_logits_cross_entropy_row_layouts(rows, V, gap, shift, dtype):
+    test_logits_cross_entropy_rows(rows, V, gap, shift, dtype)
+
+
 # chunk and tile edges of the sort by counting, several tiles of ids, the range sorted by the library; one id only, ids
 # outside the table
 @pytest.mark.parametrize("T,V,N", [(1, 5, 8), (31, 40, 64), (32, 3, 896), (33, 1, 8), (64, 1000, 1032), (65, 7, 256),

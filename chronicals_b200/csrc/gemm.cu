@@ -781,7 +781,7 @@ int choose_kernel(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool p
   const bool narrow = r128 == 1 || t128 < t256;
   const double single = narrow ? t128 : t256;
   const bool adapter = N <= 64 && !a_mn;
-  const bool long_k = r128 == 1 && !adapter && !a_mn && !b_mn && kb >= 72 && (M > 256 || N <= 1024) &&
+  const bool long_k = r128 == 1 && !adapter && !a_mn && !b_mn && kb >= 72 && (M > 256 || N <= (kb < 128 ? 1152 : 2048)) &&
                       static_cast<long long>((M + 255) / 256) * ((N + 191) / 192) <= sms / 2;
   const bool compare = pairs_possible && (r128 > 1 || adapter || long_k);
   const double pair = compare ? 1e-3 * cb_gemm2sm_cost_ns(M, N, K, a_mn, b_mn, out_bytes, sms) : 0.0;

@@ -810,9 +810,9 @@ PairPlan plan_pairs(int M, int N, int K, int a_mn, int b_mn, int out_bytes, bool
     const long long T = static_cast<long long>((M + 255) / 256) * ((N + bn - 1) / bn);
     const long long pairs = T < sms / 2 ? T : sms / 2;
     const double whole = fixed[i] + (a_mn && b_mn ? per_kb_mn : per_kb)[i] * ((T + pairs - 1) / pairs) * kb + per_mb[i] * mb;
-    // a narrower tile reads more per product, which the larger problems feel in L2 and in power; tiles that fit one round leave
-    // both to spare (696 x 120 x 18,944: 68 us with 192, 77 with 224)
-    const double handicap = T <= sms / 2 ? 0.0 : 0.12 * std::min(1.0, whole / 150.0);
+    // a narrower tile reads more per product, which the larger problems feel in L2 and in power; K-major tiles that fit one round
+    // leave both to spare (696 x 120 x 18,944: 68 us with 192, 77 with 224; 568 x 4864 x 18,944 MN-major: 105 with 256, 117 with 224)
+    const double handicap = T <= sms / 2 && !a_mn && !b_mn ? 0.0 : 0.12 * std::min(1.0, whole / 150.0);
     if (best.bn == 0 || whole * (1.0 + handicap) < best.us) best = {bn, false, whole};
     // pairs at different depths of K share no operands, which a very long K does not forgive unless most tiles are whole
     // (2624 x 3584 x 37,888: 681 us against 512); below 32 k-blocks the fixups of many small runs outweigh the estimate

@@ -158,6 +158,19 @@ def test_mxfp8_copies_of_a_matrix_and_its_transpose(R, C, pitch, shift, fmt, row
             assert torch.equal(got, qr.view(torch.uint8)) and torch.equal(scales, F8.pack_mx_scales(sr, tile))
 
 
+def test_the_copy_along_the_rows_alone_needs_no_transposing_kernel(monkeypatch):
+    from chronicals_b200.ops import ref
+    from chronicals_b200.utils import fp8_utils as F8
+
+    def refuse(*a):
+        raise AssertionError("kernel of both copies")
+    monkeypatch.setattr(ops._ext.lib(), "cb_mxfp8_quant_dual", refuse, raising=False)
+    x = torch.randn(96, 416, device=DEV, generator=_gen(5)).to(torch.bfloat16)
+    q, s, qt, st = F8.mxfp8_quantize_dual(x, "e4m3", 128, 192, True, False)
+    qr, sr = ref.mxfp8_quantize(x.float(), "e4m3")
+    assert torch.equal(q, qr.view(torch.uint8)) and torch.equal(s, F8.pack_mx_scales(sr, 128)) and qt is None and st is None
+
+
 # one chunk and several, a last chunk narrower than a tile, a vocabulary that is no multiple of 8
 @pytest.mark.parametrize("T,V,chunk", [(130, 5000, None), (130, 5000, 2048), (64, 4099, 1024), (257, 2056, 2048)])
 def test_linear_cross_entropy_chunks(T, V, chunk, monkeypatch):

@@ -947,13 +947,16 @@ int ce_split(long long rows, int V) {
   while (split < 8 && rows * split < 4LL * sm_count() && V / (2 * split) >= 4096) split *= 2;
   return split;
 }
-// In the forward pass, where a row is `nvec` 16-byte vectors, they form a cluster (a portable one has 8 at most) and meeting costs it about a microsecond:
-// long rows as above in pieces of 2048 vectors, or rows so few that they leave half the SMs without a block.  Measured, bf16,
-// one / two / four blocks a row: 16 x 32,000 6.2 / 5.4 / 4.4 us, 200 x 50,257 (one: 11 and more) 9.7 / 10.4, 400 x 16,384 6.3 / 8.1,
-// 100 x 8192 3.5 / 4.4.
+// In the forward pass, where a row is `nvec` 16-byte vectors, they form a cluster (a portable one has 8 at most) and meeting costs
+// about a microsecond: long rows as above in pieces of 2048 vectors; very long ones in pieces of 4096 also when there are many,
+// since rows that are masked leave the rest unevenly spread over one round of blocks; or rows so few that they leave half the
+// SMs without a block.  Measured, bf16, one / two / four blocks a row: 16 x 32,000 6.2 / 5.4 / 4.4 us, 200 x 50,257 (one: 11 and
+// more) 9.7 / 10.4, 400 x 16,384 6.3 / 8.1, 100 x 8192 3.5 / 4.4; 2047 x 151,936 fp32, a fifth of the rows masked, 173 / 145;
+// 1000 x 100,000 bf16, half of them, 47 / 31.
 int ce_cluster(long long rows, int nvec) {
   int split = 1;
   while (split < 8 && ((rows * split < 4LL * sm_count() && nvec / (2 * split) >= 2048) ||
+                       (rows * split < 24LL * sm_count() && nvec / (2 * split) >= 4096) ||
                        (2 * rows * split <= sm_count() && nvec >= 3072 && nvec / (2 * split) >= 512)))
     split *= 2;
   return split;
